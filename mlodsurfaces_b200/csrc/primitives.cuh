@@ -21,7 +21,13 @@ cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uin
 // temp must hold radix_temp_bytes(n) bytes.  vals and vals_alt may both be
 // nullptr to sort keys alone.
 size_t radix_temp_bytes(int64_t n);
+// Whether a sort of n items runs in one block (one launch, in place, digits
+// without differences skipped).
+bool radix_sort_is_small(int64_t n);
 cudaError_t radix_sort_pairs_u64(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
+                                 int nbits, bool* result_in_alt, void* temp, cudaStream_t s);
+// The same for 32-bit keys.
+cudaError_t radix_sort_pairs_u32(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, int64_t n,
                                  int nbits, bool* result_in_alt, void* temp, cudaStream_t s);
 
 }  // namespace mlods

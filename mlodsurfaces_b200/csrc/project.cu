@@ -1021,7 +1021,7 @@ cudaError_t launch_rule(const ProjectArgs& a, int ktype, int sm_count, cudaStrea
 // Morton key of a query on a 1024^3 grid over its tree's root box, prefixed
 // by the cloud index in the batched case.
 __global__ void query_codes_kernel(const float* __restrict__ q, int64_t n, double o0, double o1, double o2,
-                                   float inv_ext, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx)
+                                   float inv_ext, uint32_t* __restrict__ keys, uint32_t* __restrict__ idx)
 {
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1032,7 +1032,7 @@ __global__ void query_codes_kernel(const float* __restrict__ q, int64_t n, doubl
         u = fminf(fmaxf(u, 0.f), 0.99999994f);
         c[k] = uint32_t(u * 1024.f);
     }
-    uint64_t code = 0;
+    uint32_t code = 0;
     for (int b = 9; b >= 0; --b)
         code = (code << 3) | ((c[0] >> b) & 1u) | (((c[1] >> b) & 1u) << 1) | (((c[2] >> b) & 1u) << 2);
     keys[i] = code;
@@ -1183,8 +1183,8 @@ cudaError_t compute_query_order(const float* d_q, int64_t n, const double origin
                                 void* temp, cudaStream_t s)
 {
     char* t = static_cast<char*>(temp);
-    uint64_t* k0 = reinterpret_cast<uint64_t*>(t);
-    uint64_t* k1 = reinterpret_cast<uint64_t*>(t + up256(size_t(n) * 8));
+    uint32_t* k0 = reinterpret_cast<uint32_t*>(t);  // 30-bit keys
+    uint32_t* k1 = reinterpret_cast<uint32_t*>(t + up256(size_t(n) * 8));
     uint32_t* v1 = reinterpret_cast<uint32_t*>(t + 2 * up256(size_t(n) * 8));
     void* rt = t + 2 * up256(size_t(n) * 8) + up256(size_t(n) * 4);
     const float inv_ext = extent > 0.f ? 1.f / extent : 1.f;
@@ -1194,7 +1194,7 @@ cudaError_t compute_query_order(const float* d_q, int64_t n, const double origin
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     bool alt = false;
-    e = radix_sort_pairs_u64(k0, d_order, k1, v1, n, 30, &alt, rt, s);
+    e = radix_sort_pairs_u32(k0, d_order, k1, v1, n, 30, &alt, rt, s);
     if (e != cudaSuccess) return e;
     if (alt) e = cudaMemcpyAsync(d_order, v1, size_t(n) * 4, cudaMemcpyDeviceToDevice, s);
     return e;
