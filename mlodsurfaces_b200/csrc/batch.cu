@@ -93,7 +93,7 @@ int enqueue(mlods_batch_s* b, const float* d_q, int64_t total, bool timed, cudaS
     // the largest trees first, each in a launch of its own: its slice of the
     // batch order, rebased to the tree's own query indices
     unsigned int* solo_counters =
-        reinterpret_cast<unsigned int*>(b->d_stats + 8 + queue_groups(int(b->h_qclouds.size())));
+        reinterpret_cast<unsigned int*>(b->d_stats + 8 + queue_groups(int(b->h_qclouds.size())) + 1);
     for (size_t k = 0; k < b->h_solo.size(); ++k) {
         const int i = b->h_solo[k];
         ProjectArgs pa;
@@ -304,7 +304,7 @@ int mlods_batch_create(const mlods_tree* trees, int32_t n_trees, mlods_batch* ou
     }
     // statistics, a 64-bit slot counter for each launch group of
     // kQueueMaxClouds trees, a 32-bit work counter for each tree
-    const size_t n_groups = size_t(queue_groups(n_trees));
+    const size_t n_groups = size_t(queue_groups(n_trees)) + 1;
     b->stats_bytes = (8 * sizeof(int64_t) + n_groups * sizeof(uint64_t) + size_t(n_trees) * sizeof(unsigned int) +
                       255) / 256 * 256;
     cudaError_t e = cudaMalloc(&b->d_offsets, size_t(n_trees + 1) * sizeof(int64_t));

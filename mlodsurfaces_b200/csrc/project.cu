@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "primitives.cuh"
 #include "project.cuh"
@@ -788,6 +789,267 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
     }
 }
 
+// ---- two nodes per lane ----------------------------------------------------
+// The wide walk pops up to 64 nodes a round: two groups of whole sibling ranges
+// of at most 32 nodes, lane l evaluating node l of each.  The pop, the scan and
+// the loop are paid once for twice the nodes and a query's chain of rounds is
+// half as long, which bounds calls of a few thousand queries: 1,000 queries,
+// 10 iterations 381 -> 204 us, 10,000 960 -> 850 us.  Calls that fill the GPU
+// gain less (100k 11.9 -> 9.9 ms, 2M four-Gaussian 245 -> 218 ms): there the
+// node loads keep the L1 data path two thirds busy, 2.1 wavefronts a visit.
+// 4 blocks per SM (128 registers) against 5 / 6 / 7: 218 / 229 / 238 / 255 ms,
+// since every resident warp's stack takes L1 away from the nodes.
+
+template <int CAP>
+struct WideStack {
+    uint2 h[CAP];   // {first, count | flags}
+    float4 v[CAP];  // {f, A, dP, g}
+};
+// Above this many ranges the walk pops the top one only (depth first), which
+// adds at most 7 ranges a level for 12 levels and a multi-point leaf's: with the
+// 64 a full round can push, the stack cannot overflow.
+template <int CAP>
+struct WideLimit {
+    static constexpr int kPop = CAP - 64 - (7 * kMaxTreeDepth + 8);
+    static_assert(kPop > 32, "stack too small for a full round");
+};
+
+// v + the value o lanes below, where there is one
+__device__ __forceinline__ int add_from_below(int v, int o)
+{
+    int r;
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .s32 t;\n shfl.sync.up.b32 t|p, %1, %2, 0, 0xffffffff;\n"
+        " @p add.s32 t, t, %1;\n @!p mov.s32 t, %1;\n mov.s32 %0, t;\n}"
+        : "=r"(r)
+        : "r"(v), "r"(o));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float v)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// A value of each of the lane's two nodes.  Plain scalar arithmetic: packing the
+// nodes' loaded components into register pairs costs the moves that the packed
+// instructions save (226 against 232 ms on the precision workload).
+struct Two {
+    float x, y;
+};
+__device__ __forceinline__ Two two(float x, float y) { return Two{x, y}; }
+__device__ __forceinline__ Two operator+(Two a, Two b) { return Two{a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ Two operator-(Two a, float b) { return Two{a.x - b, a.y - b}; }
+__device__ __forceinline__ Two operator-(Two a, Two b) { return Two{a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ Two operator*(Two a, Two b) { return Two{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ Two operator*(float a, Two b) { return Two{a * b.x, a * b.y}; }
+__device__ __forceinline__ Two fma2(Two a, Two b, Two c) { return Two{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+
+template <int KTYPE, int NSIG, int RULE, int CAP>
+__device__ __forceinline__ void project_wide(const CloudArgs& c, uint32_t my_q, WideStack<CAP>& st, WalkStats& ws)
+{
+    const bool gpu_rule = RULE < 0 ? c.rule == MLODS_BLEND_GPU : RULE == MLODS_BLEND_GPU;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t le_mask = lane == 31 ? kFull : ((2u << lane) - 1u);
+    const float4* __restrict__ ngeom = c.nodes.geom;
+    const float4* __restrict__ npm = c.nodes.pm;
+    const float4* __restrict__ nnc = c.nodes.nc;
+    const float4* __restrict__ naux = c.nodes.aux;
+    const float cutoff = c.cutoff;
+    const int min_depth = c.min_depth;
+    double qd[3] = {double(c.q_in[3 * int64_t(my_q)]) - c.o0, double(c.q_in[3 * int64_t(my_q) + 1]) - c.o1,
+                    double(c.q_in[3 * int64_t(my_q) + 2]) - c.o2};
+    float nrm[3] = {0.f, 0.f, 0.f};
+    bool failed = false, stop = false;
+    for (int it = 0; it < c.n_iter && !stop; ++it) {
+        const float fx = float(qd[0]), fy = float(qd[1]), fz = float(qd[2]);
+        ++ws.iterations;
+        // a NaN iterate would open every node and fail; it fails at once
+        if (!(fx == fx && fy == fy && fz == fz)) {
+            failed = true;
+            break;
+        }
+        Two acc[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) acc[k] = two(0.f, 0.f);
+        int top = 1;
+        if (lane == 0) {
+            st.h[0] = make_uint2(0u, 1u | kEntNoBlend);
+            st.v[0] = make_float4(1.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+        while (top > 0) {
+            // ---- pop sibling ranges from the top: group 0 as many as fill 32
+            // lanes, group 1 the next as many as fill 32 again
+            // (the top 16 ranges hold 64 nodes or nearly)
+            const int avail = min(top > WideLimit<CAP>::kPop ? 1 : top, 16);
+            const int idx = top - 1 - lane;
+            const int cn = lane < avail ? int(st.h[idx].y & kEntCount) : 0x1000000;
+            int incl = cn;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) incl = add_from_below(incl, o);
+            const int n0 = __popc(__ballot_sync(kFull, incl <= 32));
+            const bool partial = n0 == 0;  // top range wider than a warp (multi-point leaf)
+            int tot0 = 32, tot1 = 0, n01 = 0;
+            uint32_t heads0 = 1u, heads1 = 0u;
+            if (!partial) {
+                tot0 = __shfl_sync(kFull, incl, n0 - 1);
+                n01 = __popc(__ballot_sync(kFull, incl <= tot0 + 32));
+                tot1 = __shfl_sync(kFull, incl, n01 - 1) - tot0;
+                const int start = incl - cn;
+                heads0 = __reduce_or_sync(kFull, lane < n0 ? 1u << start : 0u);
+                heads1 = __reduce_or_sync(kFull, lane >= n0 && lane < n01 ? 1u << (start - tot0) : 0u);
+            }
+            const uint32_t hb0 = heads0 & le_mask, hb1 = heads1 & le_mask;
+            const int s0 = 31 - __clz(hb0), s1 = 31 - __clz(hb1);
+            // (an empty group 1 reads the top entry)
+            const int slot0 = top - __popc(hb0), slot1 = hb1 ? top - n0 - __popc(hb1) : top - 1;
+            const uint2 E0 = st.h[slot0], E1 = st.h[slot1];
+            const float4 V0 = st.v[slot0], V1 = st.v[slot1];
+            const bool act0 = lane < tot0, act1 = lane < tot1;
+            const int len0 = partial ? 32 : int(E0.y & kEntCount), len1 = int(E1.y & kEntCount);
+            // lanes past the last range repeat its last node
+            const uint32_t node0 = E0.x + uint32_t(min(lane - s0, len0 - 1));
+            const uint32_t node1 = E1.x + uint32_t(min(lane - s1, len1 - 1));
+            const int old_top = top;
+            top -= n01;
+            ws.lane_visits += uint32_t(tot0 + tot1);
+            ++ws.rounds;
+
+            // ---- evaluate two nodes per lane
+            const float4 ga = __ldg(ngeom + node0), gb = __ldg(ngeom + node1);
+            const float4 pa = __ldg(npm + node0), pb = __ldg(npm + node1);
+            const float4 xa = __ldg(naux + node0), xb = __ldg(naux + node1);
+            const float4 na = __ldg(nnc + node0), nb = __ldg(nnc + node1);
+            const Two cr = cutoff * two(ga.w, gb.w);
+            const Two cx = two(ga.x, gb.x) - fx, cy = two(ga.y, gb.y) - fy, cz = two(ga.z, gb.z) - fz;
+            const Two dd = fma2(cx, cx, fma2(cy, cy, cz * cz));
+            const Two dist = two(sqrtf(dd.x), sqrtf(dd.y));
+            const Two mdP = dist - cr;  // -(cutoff r - dist)
+            const Two m2 = two(pa.w, pb.w);
+            Two beta, kcon;
+            {
+                const bool bl0 = act0 && !(E0.y & kEntNoBlend), bl1 = act1 && !(E1.y & kEntNoBlend);
+                const Two dP = two(V0.z, V1.z);
+                const Two den = dP + two(fmaxf(mdP.x, 0.f), fmaxf(mdP.y, 0.f));
+                const Two t = (kPiRef * dP) * two(rcp_fast(den.x), rcp_fast(den.y));
+                const Two h = two(__cosf(t.x), __cosf(t.y));
+                beta = fma2(two(-0.5f, -0.5f), h, two(0.5f, 0.5f));
+                kcon = fma2(two(0.5f, 0.5f), h, two(0.5f, 0.5f)) * two(V0.w, V1.w);  // (1 - beta) g
+                if (gpu_rule) kcon = kcon * m2;
+                beta = two(bl0 ? beta.x : 1.f, bl1 ? beta.y : 1.f);
+                kcon = two(bl0 ? kcon.x : 0.f, bl1 ? kcon.y : 0.f);
+            }
+            // segmented sums over the ranges (blend ranges hold <= 8 lanes)
+            {
+                const int rem0 = s0 + len0 - lane, rem1 = s1 + len1 - lane;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const float u0 = __shfl_down_sync(kFull, kcon.x, o), u1 = __shfl_down_sync(kFull, kcon.y, o);
+                    if (o < rem0) kcon.x += u0;
+                    if (o < rem1) kcon.y += u1;
+                }
+            }
+            const Two K = two(__shfl_sync(kFull, kcon.x, s0), __shfl_sync(kFull, kcon.y, s1));
+            Two f = two(V0.x, V1.x) * beta;
+            const Two A = two(V0.y, V1.y) + K;
+            if (!gpu_rule) {  // the CPU rule weighs only the last point of a multi-point leaf
+                if ((E0.y & kEntLastOnly) && (partial || node0 != E0.x + uint32_t(len0) - 1u)) f.x = 0.f;
+                if ((E1.y & kEntLastOnly) && node1 != E1.x + uint32_t(len1) - 1u) f.y = 0.f;
+            }
+            // the distance beyond which a node ends the walk: any for a leaf;
+            // none for what is opened whatever its distance, the points of a
+            // multi-point leaf and the children of a node above min_depth
+            const uint32_t info0 = __float_as_uint(xa.z), info1 = __float_as_uint(xb.z);
+            const bool all0 = (info0 & kLeafBit) ? (info0 & kMultiBit) != 0 : node_depth(info0) < min_depth;
+            const bool all1 = (info1 & kLeafBit) ? (info1 & kMultiBit) != 0 : node_depth(info1) < min_depth;
+            const float thr0 = all0 ? INFINITY : ((info0 & kLeafBit) ? -1.f : cr.x);
+            const float thr1 = all1 ? INFINITY : ((info1 & kLeafBit) ? -1.f : cr.y);
+            const bool far0 = dist.x > thr0, far1 = dist.y > thr1;
+            const bool push0 = act0 && !far0, push1 = act1 && !far1;
+
+            const Two px = two(pa.x, pb.x) - fx, py = two(pa.y, pb.y) - fy, pz = two(pa.z, pb.z) - fz;
+            const Two d2 = fma2(px, px, fma2(py, py, pz * pz));
+            const Two w = two(weight_n<KTYPE, NSIG>(c.kc, d2.x), weight_n<KTYPE, NSIG>(c.kc, d2.y));
+            const uint32_t cnt0 = node_count(info0), cnt1 = node_count(info1);
+            const Two fw = f * w;
+            {
+                // an opened node adds nothing (its moments are finite: a node
+                // without mass has none, and leaves its ancestors none either)
+                Two coef = fma2(f, w, A);
+                coef = two(act0 && far0 ? coef.x : 0.f, act1 && far1 ? coef.y : 0.f);
+                const Two nx = two(na.x, nb.x), ny = two(na.y, nb.y), nz = two(na.z, nb.z);
+                const Two cm = coef * m2;
+                acc[0] = acc[0] + cm;
+                acc[1] = fma2(coef, nx, acc[1]);
+                acc[2] = fma2(coef, ny, acc[2]);
+                acc[3] = fma2(coef, nz, acc[3]);
+                acc[4] = fma2(cm, px, acc[4]);
+                acc[5] = fma2(cm, py, acc[5]);
+                acc[6] = fma2(cm, pz, acc[6]);
+                acc[7] = fma2(coef, fma2(px, nx, fma2(py, ny, fma2(pz, nz, two(na.w, nb.w)))), acc[7]);
+                acc[8] = fma2(coef, fma2(d2, m2, two(xa.x, xb.x)), acc[8]);
+            }
+            // ---- push child ranges (every lane has read its entries)
+            __syncwarp();
+            if (partial && lane == 0) {
+                uint2 rest = st.h[old_top - 1];
+                rest.x += 32u;
+                rest.y -= 32u;
+                st.h[old_top - 1] = rest;
+            }
+            const uint32_t pm0 = __ballot_sync(kFull, push0), pm1 = __ballot_sync(kFull, push1);
+            if (push0) {
+                const int pos = top + __popc(pm0 & lt_mask);
+                const uint32_t flags = all0 ? kEntNoBlend | ((info0 & kLeafBit) && !gpu_rule ? kEntLastOnly : 0u) : 0u;
+                st.h[pos] = make_uint2(__float_as_uint(xa.y), cnt0 | flags);
+                st.v[pos] = make_float4(f.x, A.x, -mdP.x, fw.x * rcp_fast(gpu_rule ? m2.x : float(cnt0)));
+            }
+            top += __popc(pm0);
+            if (push1) {
+                const int pos = top + __popc(pm1 & lt_mask);
+                const uint32_t flags = all1 ? kEntNoBlend | ((info1 & kLeafBit) && !gpu_rule ? kEntLastOnly : 0u) : 0u;
+                st.h[pos] = make_uint2(__float_as_uint(xb.y), cnt1 | flags);
+                st.v[pos] = make_float4(f.y, A.y, -mdP.y, fw.y * rcp_fast(gpu_rule ? m2.y : float(cnt1)));
+            }
+            top += __popc(pm1);
+            if (top > ws.max_top) ws.max_top = top;
+            __syncwarp();
+        }
+        float sv[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) sv[k] = warp_sum_f(acc[k].x + acc[k].y);
+        double xr[3] = {0.0, 0.0, 0.0};
+        if (!fit_sphere(sv, double(c.step_max), gpu_rule, xr, nrm)) {
+            failed = true;
+            break;
+        }
+        qd[0] = double(fx) + xr[0];
+        qd[1] = double(fy) + xr[1];
+        qd[2] = double(fz) + xr[2];
+        if (c.conv_mode == MLODS_CONVERGE_EXACT) {
+            stop = float(qd[0]) == fx && float(qd[1]) == fy && float(qd[2]) == fz;
+        } else if (c.conv_mode == MLODS_CONVERGE_TOL) {
+            stop = xr[0] * xr[0] + xr[1] * xr[1] + xr[2] * xr[2] < double(c.conv_tol) * double(c.conv_tol);
+        }
+    }
+    ws.visits = ws.lane_visits;
+    if (lane == 0) {
+        float* op = c.out_p + 3 * int64_t(my_q);
+        float* on = c.out_n + 3 * int64_t(my_q);
+        // on failure (Fastapss.cu:385-391) the point stays where the failing
+        // iteration started and the normal is zero
+        op[0] = float(c.local_out ? qd[0] : qd[0] + c.o0);
+        op[1] = float(c.local_out ? qd[1] : qd[1] + c.o1);
+        op[2] = float(c.local_out ? qd[2] : qd[2] + c.o2);
+        on[0] = failed ? 0.f : nrm[0];
+        on[1] = failed ? 0.f : nrm[1];
+        on[2] = failed ? 0.f : nrm[2];
+    }
+}
+
 // Projects the nq (<= QPW) queries qi[0..nq) of one tree together (the
 // general walk for one query per warp, the packed form for two or four).
 template <int KTYPE, int NSIG, int RULE, int CAP, int QPW, bool PRUNE = false, bool EARLY_NC = true>
@@ -842,6 +1104,25 @@ struct WalkShape {
     static constexpr int kMinBlocks = QPW == 1 ? kProjectMinBlocks : (QPW == 2 ? kProjectPairMinBlocks : 5);
     static constexpr int kCap = QPW == 1 ? kProjectStackCap : kProjectPairStackCap;
 };
+
+template <int KTYPE, int NSIG, int RULE>
+__global__ void __launch_bounds__(kProjectThreads, kWideMinBlocks) mlod_wide_kernel(ProjectArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    WideStack<kWideCap>& st = reinterpret_cast<WideStack<kWideCap>*>(smem_raw)[threadIdx.x >> 5];
+    WarpTotals tot;
+    for (;;) {
+        unsigned int qs = 0;
+        if (lane == 0) qs = atomicAdd(a.counter, 1u);
+        qs = __shfl_sync(kFull, qs, 0);
+        if (int64_t(qs) >= a.nq) break;
+        WalkStats ws;
+        project_wide<KTYPE, NSIG, RULE, kWideCap>(a.cloud, a.order ? __ldg(a.order + qs) - a.order_base : qs, st, ws);
+        tot.add(ws, 1);
+    }
+    tot.flush(a.stats);
+}
 
 template <int KTYPE, int NSIG, int RULE, int QPW, bool PRUNE>
 __global__ void __launch_bounds__(kProjectThreads, WalkShape<QPW>::kMinBlocks) mlod_project_kernel(ProjectArgs a)
@@ -908,6 +1189,22 @@ inline int walk_spec_id(const CloudArgs& c)
     return (c.rule == MLODS_BLEND_GPU ? 0 : 1) * 9 + k;
 }
 
+template <int RULE>
+__device__ __forceinline__ void walk_wide_k(int k, const CloudArgs& c, uint32_t q, WideStack<kWideCap>& st, WalkStats& ws)
+{
+    switch (k) {
+    case 0: project_wide<MLODS_GAUSSIAN, 0, RULE, kWideCap>(c, q, st, ws); break;
+    case 1: project_wide<MLODS_SINGULAR, 0, RULE, kWideCap>(c, q, st, ws); break;
+    case 2: project_wide<MLODS_GAUSSIAN_MULTIPLE, 2, RULE, kWideCap>(c, q, st, ws); break;
+    case 3: project_wide<MLODS_GAUSSIAN_MULTIPLE, 3, RULE, kWideCap>(c, q, st, ws); break;
+    case 4: project_wide<MLODS_GAUSSIAN_MULTIPLE, 4, RULE, kWideCap>(c, q, st, ws); break;
+    case 5: project_wide<MLODS_GAUSSIAN_MULTIPLE, 5, RULE, kWideCap>(c, q, st, ws); break;
+    case 6: project_wide<MLODS_GAUSSIAN_MULTIPLE, 6, RULE, kWideCap>(c, q, st, ws); break;
+    case 7: project_wide<MLODS_GAUSSIAN_MULTIPLE, 8, RULE, kWideCap>(c, q, st, ws); break;
+    default: project_wide<MLODS_GAUSSIAN_MULTIPLE, 0, RULE, kWideCap>(c, q, st, ws); break;
+    }
+}
+
 template <int RULE, int CAP, int QPW>
 __device__ __forceinline__ void walk_k(int k, const CloudArgs& c, const uint32_t (&qi)[QPW], int nq,
                                        WarpStack<CAP, QPW>& st, WalkStats& ws)
@@ -931,14 +1228,16 @@ __device__ __forceinline__ void walk_k(int k, const CloudArgs& c, const uint32_t
 // any moment share node records in L1 and L2), finds their cloud by binary
 // search over the line and walks them with the cloud's own specialisation;
 // the kernel is compiled with the schedule's registers and blocks per SM.
-template <int QPW>
-__global__ void __launch_bounds__(kProjectThreads, WalkShape<QPW>::kMinBlocks)
+template <int QPW, bool WIDE>
+__global__ void __launch_bounds__(kProjectThreads, WIDE ? kWideMinBlocks : WalkShape<QPW>::kMinBlocks)
     mlod_queue_kernel(const __grid_constant__ QueueLaunch p)
 {
+    static_assert(!WIDE || QPW == 1, "the wide walk serves one query");
     constexpr int CAP = WalkShape<QPW>::kCap;
+    using Stack = std::conditional_t<WIDE, WideStack<kWideCap>, WarpStack<CAP, QPW>>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
-    WarpStack<CAP, QPW>& st = reinterpret_cast<WarpStack<CAP, QPW>*>(smem_raw)[threadIdx.x >> 5];
+    Stack& st = reinterpret_cast<Stack*>(smem_raw)[threadIdx.x >> 5];
     WarpTotals tot;
     for (;;) {
         unsigned long long v = 0;
@@ -964,8 +1263,13 @@ __global__ void __launch_bounds__(kProjectThreads, WalkShape<QPW>::kMinBlocks)
         const CloudArgs& c = p.clouds[ci];
         const int sp = p.spec[ci];
         WalkStats ws;
-        if (sp < 9) walk_k<MLODS_BLEND_GPU, CAP, QPW>(sp, c, qi, nq, st, ws);
-        else walk_k<MLODS_BLEND_CPU, CAP, QPW>(sp - 9, c, qi, nq, st, ws);
+        if constexpr (WIDE) {
+            if (sp < 9) walk_wide_k<MLODS_BLEND_GPU>(sp, c, qi[0], st, ws);
+            else walk_wide_k<MLODS_BLEND_CPU>(sp - 9, c, qi[0], st, ws);
+        } else {
+            if (sp < 9) walk_k<MLODS_BLEND_GPU, CAP, QPW>(sp, c, qi, nq, st, ws);
+            else walk_k<MLODS_BLEND_CPU, CAP, QPW>(sp - 9, c, qi, nq, st, ws);
+        }
         tot.add(ws, nq);
     }
     tot.flush(p.stats);
@@ -987,6 +1291,18 @@ int64_t persistent_grid(Kern kern, size_t smem, int64_t work_warps, int sm_count
 template <int KTYPE, int NSIG, int RULE, int QPW>
 cudaError_t launch_typed(const ProjectArgs& a, int sm_count, cudaStream_t s)
 {
+    if constexpr (QPW == 1) {
+        if (walks_wide(a.cloud)) {
+            auto wide = mlod_wide_kernel<KTYPE, NSIG, RULE>;
+            const size_t smem = size_t(kProjectThreads / 32) * sizeof(WideStack<kWideCap>);
+            cudaError_t e = cudaSuccess;
+            const int64_t grid = persistent_grid(wide, smem, a.nq, sm_count, &e);
+            if (e != cudaSuccess) return e;
+            wide<<<unsigned(grid), kProjectThreads, smem, s>>>(a);
+            note_launch();
+            return cudaGetLastError();
+        }
+    }
     constexpr int CAP = WalkShape<QPW>::kCap;
     // kernel-weight pruning is a variant of its own (four queries per warp
     // has none), so the default walk carries none of its code
@@ -1104,26 +1420,31 @@ cudaError_t launch_mlod_project(const ProjectArgs& a, int ktype, int rule, int s
 
 namespace
 {
-template <int QPW>
-cudaError_t launch_queue_typed(const QueueArgs& a, int sm_count, int grid_pct, cudaStream_t s)
+// The clouds `which` of a batch, in groups of one launch each; uses a counter a
+// group from `counters` on.
+template <int QPW, bool WIDE>
+cudaError_t launch_queue_typed(const QueueArgs& a, const std::vector<int>& which, unsigned long long* counters,
+                               int sm_count, int grid_pct, cudaStream_t s)
 {
     constexpr int CAP = WalkShape<QPW>::kCap;
-    const size_t smem = size_t(kProjectThreads / 32) * sizeof(WarpStack<CAP, QPW>);
-    const int n_groups = queue_groups(a.n_clouds);
+    const size_t smem =
+        size_t(kProjectThreads / 32) * (WIDE ? sizeof(WideStack<kWideCap>) : sizeof(WarpStack<CAP, QPW>));
+    const int n_groups = queue_groups(int(which.size()));
     for (int g = 0; g < n_groups; ++g) {
-        const int c0 = g * kQueueMaxClouds, nc = std::min(kQueueMaxClouds, a.n_clouds - c0);
+        const int c0 = g * kQueueMaxClouds, nc = std::min(kQueueMaxClouds, int(which.size()) - c0);
         QueueLaunch p;
         std::memset(&p, 0, sizeof p);
         p.order = a.order;
-        p.counter = a.counters + g;
+        p.counter = counters + g;
         p.stats = a.stats;
         p.n = nc;
         std::vector<int> idx(static_cast<size_t>(nc));
         for (int i = 0; i < nc; ++i) {
             idx[size_t(i)] = i;
-            p.clouds[i] = a.clouds[c0 + i];
-            p.base[i] = a.base[c0 + i];
-            p.len[i] = a.len[c0 + i];
+            const int c = which[size_t(c0 + i)];
+            p.clouds[i] = a.clouds[c];
+            p.base[i] = a.base[c];
+            p.len[i] = a.len[c];
             p.spec[i] = walk_spec_id(p.clouds[i]);
         }
         // the clouds with the most work first, so that the launch ends on
@@ -1149,10 +1470,10 @@ cudaError_t launch_queue_typed(const QueueArgs& a, int sm_count, int grid_pct, c
         p.v_total = v;
         if (v == 0) continue;
         cudaError_t e = cudaSuccess;
-        int64_t grid = persistent_grid(mlod_queue_kernel<QPW>, smem, (v + QPW - 1) / QPW, sm_count, &e);
+        int64_t grid = persistent_grid(mlod_queue_kernel<QPW, WIDE>, smem, (v + QPW - 1) / QPW, sm_count, &e);
         if (e != cudaSuccess) return e;
         if (grid_pct > 0 && grid_pct < 100) grid = std::max<int64_t>(1, grid * grid_pct / 100);
-        mlod_queue_kernel<QPW><<<unsigned(grid), kProjectThreads, smem, s>>>(p);
+        mlod_queue_kernel<QPW, WIDE><<<unsigned(grid), kProjectThreads, smem, s>>>(p);
         note_launch();
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -1163,14 +1484,23 @@ cudaError_t launch_queue_typed(const QueueArgs& a, int sm_count, int grid_pct, c
 
 cudaError_t launch_mlod_queue(const QueueArgs& a, int queries_per_warp, int sm_count, int grid_pct, cudaStream_t s)
 {
-    if (queries_per_warp == 2) return launch_queue_typed<2>(a, sm_count, grid_pct, s);
-    return launch_queue_typed<1>(a, sm_count, grid_pct, s);
+    // each cloud walks as a launch of its own would: the clouds of one query
+    // per warp that walk wide in a launch apart from those that do not
+    std::vector<int> wide, rest;
+    for (int i = 0; i < a.n_clouds; ++i)
+        (queries_per_warp != 2 && walks_wide(a.clouds[i]) ? wide : rest).push_back(i);
+    cudaError_t e = cudaSuccess;
+    if (!wide.empty()) e = launch_queue_typed<1, true>(a, wide, a.counters, sm_count, grid_pct, s);
+    if (e != cudaSuccess || rest.empty()) return e;
+    unsigned long long* counters = a.counters + queue_groups(int(wide.size()));
+    if (queries_per_warp == 2) return launch_queue_typed<2, false>(a, rest, counters, sm_count, grid_pct, s);
+    return launch_queue_typed<1, false>(a, rest, counters, sm_count, grid_pct, s);
 }
 
 int64_t project_resident_queries(int queries_per_warp, int sm_count)
 {
     const int per_sm = queries_per_warp == 4 ? WalkShape<4>::kMinBlocks
-                                             : (queries_per_warp == 2 ? WalkShape<2>::kMinBlocks : WalkShape<1>::kMinBlocks);
+                                             : (queries_per_warp == 2 ? WalkShape<2>::kMinBlocks : kWideMinBlocks);
     return int64_t(per_sm) * (kProjectThreads / 32) * queries_per_warp * sm_count;
 }
 

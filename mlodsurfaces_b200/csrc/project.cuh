@@ -30,6 +30,11 @@ constexpr int kProjectStackCap = MLODS_PROJECT_STACK_CAP;    // sibling ranges p
 constexpr int kProjectPairMinBlocks = MLODS_PROJECT_PAIR_MIN_BLOCKS;
 constexpr int kProjectPairStackCap = MLODS_PROJECT_PAIR_STACK_CAP;
 
+// the wide walk (one query per warp, two nodes a lane): 128 registers, a stack
+// of whole 64-node rounds (24 bytes a range)
+constexpr int kWideMinBlocks = 4;
+constexpr int kWideCap = 288;
+
 // One tree and its projection settings, plus the query buffers it serves.
 struct CloudArgs {
     NodeArrays nodes;
@@ -49,6 +54,14 @@ struct CloudArgs {
     int qpw;                // the tree's walk schedule (queries per warp) for launches of its own
     float prune_thr;        // > 0: kernel-weight pruning threshold (prune_tol * w(0) * mean sample area)
 };
+
+// Whether a one-query-per-warp projection takes the wide walk.  Not with one
+// iteration: that is the projection behind the dual-contouring field and the
+// cell grids, whose signs and cells are whole numbers that follow the float
+// sums of the narrow walk bit for bit; and not with pruning, which is a variant
+// of the narrow walk.  The rule looks at nothing that a batch or a server
+// changes, so a query's result does not depend on what it is projected with.
+inline bool walks_wide(const CloudArgs& c) { return c.n_iter >= 2 && !(c.prune_thr > 0.f); }
 
 struct ProjectArgs {
     CloudArgs cloud;
@@ -91,6 +104,8 @@ constexpr int kQueueBySpecialisation = 1;
 // value in the kernel's parameters (within the 32 KB parameter limit); a
 // batch of more clouds runs as consecutive launches of up to this many.
 constexpr int kQueueMaxClouds = 80;
+// (clouds that walk wide and clouds that do not are grouped apart: a mixed
+// batch uses at most one group, and one counter, more)
 inline int queue_groups(int n_clouds) { return (n_clouds + kQueueMaxClouds - 1) / kQueueMaxClouds; }
 
 // The queue kernel over every group of clouds (usually one launch); every

@@ -109,7 +109,7 @@ inline size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 // groups), then a 32-bit work counter for each piece that runs in a launch
 // of its own
 constexpr int kMaxServeGroups = 64;
-constexpr size_t kStatsBytes = 8 * sizeof(int64_t) + kMaxServeGroups * sizeof(uint64_t) +
+constexpr size_t kStatsBytes = 8 * sizeof(int64_t) + (kMaxServeGroups + 1) * sizeof(uint64_t) +
                                size_t(kMaxServeGroups) * kQueueMaxClouds * sizeof(unsigned int);
 // A piece of at least this many times the queries the walk holds in flight
 // on the whole GPU runs in a launch of its own (the single-tree kernel, whose
@@ -238,7 +238,7 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
         const int64_t solo_min = kSoloFill * project_resident_queries(qpw, sm);
         std::vector<CloudArgs> qclouds;
         std::vector<int64_t> qbase, qlen;
-        unsigned int* solo_counters = reinterpret_cast<unsigned int*>(w.d_stats + 8 + kMaxServeGroups);
+        unsigned int* solo_counters = reinterpret_cast<unsigned int*>(w.d_stats + 8 + kMaxServeGroups + 1);
         int n_solo = 0;
         for (size_t i = 0; i < nc && e == cudaSuccess; ++i) {
             const int64_t len = w.h_offsets[i + 1] - w.h_offsets[i];
