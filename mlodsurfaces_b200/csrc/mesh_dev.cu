@@ -170,7 +170,7 @@ struct Buf {
     Buf() = default;
     Buf(const Buf&) = delete;
     Buf& operator=(const Buf&) = delete;
-    ~Buf() { cudaFree(p); }
+    ~Buf() { durable_free(p); }
     void swap(Buf& o)
     {
         std::swap(p, o.p);
@@ -179,10 +179,10 @@ struct Buf {
     int need(size_t bytes)
     {
         if (bytes <= cap) return MLODS_OK;
-        cudaFree(p);
+        durable_free(p);
         p = nullptr;
         cap = 0;
-        MLODS_CUDA(cudaMalloc(&p, bytes));
+        MLODS_CUDA(durable_alloc(&p, bytes));
         cap = bytes;
         return MLODS_OK;
     }

@@ -142,6 +142,15 @@ int sm_count_for_current_device();
 // Stream-ordered scratch memory from the library's pool on the current device.
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 cudaError_t scratch_free(void* p, cudaStream_t s);
+// Memory that outlives the call, from the same pool: ready for every stream on
+// return, freed once everything on its device that may use it has run.
+cudaError_t durable_alloc(void** p, size_t bytes);
+cudaError_t durable_free(void* p);
+template <typename T>
+cudaError_t durable_alloc(T** p, size_t bytes)
+{
+    return durable_alloc(reinterpret_cast<void**>(p), bytes);
+}
 
 // Makes `dev` the calling thread's current device for the life of the guard
 // and restores the previous one afterwards (a tree, batch or server holds

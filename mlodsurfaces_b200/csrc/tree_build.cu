@@ -481,7 +481,7 @@ __global__ void sorted_points_kernel(int64_t n, const uint32_t* __restrict__ per
 
 inline size_t al(size_t v) { return (v + 255) / 256 * 256; }
 
-// A simple bump allocator over one cudaMalloc'd block of build temporaries.
+// A simple bump allocator over one block of build temporaries.
 struct Bump {
     char* base = nullptr;
     size_t off = 0, cap = 0;
@@ -498,15 +498,15 @@ struct Bump {
 
 void free_tree_device(mlods_tree_s* T)
 {
-    cudaFree(T->nodes.geom);
-    cudaFree(T->d_node_head);
-    cudaFree(T->d_codes);
-    cudaFree(T->d_perm);
-    cudaFree(T->d_area);
-    cudaFree(T->d_spts);
-    cudaFree(T->d_snrm);
-    cudaFree(T->d_wspts);
-    cudaFree(T->d_bounds);
+    durable_free(T->nodes.geom);
+    durable_free(T->d_node_head);
+    durable_free(T->d_codes);
+    durable_free(T->d_perm);
+    durable_free(T->d_area);
+    durable_free(T->d_spts);
+    durable_free(T->d_snrm);
+    durable_free(T->d_wspts);
+    durable_free(T->d_bounds);
     T->nodes = NodeArrays{};
     T->d_node_head = nullptr;
     T->d_codes = nullptr;
@@ -535,7 +535,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     // ---- root box (CPUUtils.cpp:571-579)
     const int nbb = int(std::min<int64_t>(1024, (n + kThreads - 1) / kThreads));
     float* d_bb = nullptr;
-    MLODS_CUDA(cudaMalloc(&d_bb, size_t(nbb) * 6 * sizeof(float) + sizeof(int)));
+    MLODS_CUDA(scratch_alloc(reinterpret_cast<void**>(&d_bb), size_t(nbb) * 6 * sizeof(float) + sizeof(int), s));
     int* d_bad = reinterpret_cast<int*>(d_bb + size_t(nbb) * 6);
     std::vector<float> hbb(size_t(nbb) * 6);
     int h_bad = 0;
@@ -548,7 +548,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     if (e == cudaSuccess) e = cudaMemcpyAsync(hbb.data(), d_bb, hbb.size() * sizeof(float), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_bb);
+    scratch_free(d_bb, s);
     if (e != cudaSuccess) return cuda_fail(e, "tree build: bbox", __FILE__, __LINE__);
     if (h_bad) {
         set_last_error("tree build: non-finite point coordinates");
@@ -618,7 +618,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
         need += al(size_t(ncounts) * 4) + al(64 * 8);
         need += std::max(radix_temp_bytes(n), scan_temp_bytes(ncounts));
         bump.cap = need;
-        MLODS_CUDA(cudaMalloc(&bump.base, need));
+        MLODS_CUDA(scratch_alloc(reinterpret_cast<void**>(&bump.base), need, s));
     }
     double* d_splits = bump.take<double>(size_t(3 * split_stride));
     uint64_t* d_k0 = bump.take<uint64_t>(size_t(n));
@@ -633,7 +633,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     void* d_tmp = bump.base + bump.off;
 
     auto fail = [&](cudaError_t err, const char* what) {
-        cudaFree(bump.base);
+        scratch_free(bump.base, s);
         return cuda_fail(err, what, __FILE__, __LINE__);
     };
 #define BUILD_CHECK(call, what)                          \
@@ -642,7 +642,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
         if (_e2 != cudaSuccess) return fail(_e2, what);  \
     } while (0)
 
-    BUILD_CHECK(cudaMalloc(&T->d_bounds, size_t(3 * bound_stride) * sizeof(float)), "alloc bounds");
+    BUILD_CHECK(durable_alloc(&T->d_bounds, size_t(3 * bound_stride) * sizeof(float)), "alloc bounds");
     T->bounds_stride = bound_stride;
     BUILD_CHECK(cudaMemcpyAsync(T->d_bounds, hb.data(), hb.size() * sizeof(float), cudaMemcpyHostToDevice, s),
                 "upload bounds");
@@ -690,7 +690,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     char* nodebuf = nullptr;
     size_t nodebytes = al(size_t(nn) * 4) * 6 + al(size_t(nn)) * 2 + al(size_t(nn) * 72) + al(size_t(D + 2) * 8) +
                        scan_temp_bytes(nn) + 256;
-    BUILD_CHECK(cudaMalloc(&nodebuf, nodebytes), "alloc node temporaries");
+    BUILD_CHECK(scratch_alloc(reinterpret_cast<void**>(&nodebuf), nodebytes, s), "alloc node temporaries");
     Bump nbm;
     nbm.base = nodebuf;
     nbm.cap = nodebytes;
@@ -706,7 +706,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     int64_t* d_lvloff = nbm.take<int64_t>(size_t(D + 2));
     void* d_ntmp = nbm.base + nbm.off;
     auto fail2 = [&](cudaError_t err, const char* what) {
-        cudaFree(nodebuf);
+        scratch_free(nodebuf, s);
         return fail(err, what);
     };
 #define NODE_CHECK(call, what)                            \
@@ -731,7 +731,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     note_launch();
     NODE_CHECK(cudaGetLastError(), "links");
 
-    MLODS_CUDA(cudaMalloc(&T->d_area, size_t(n) * sizeof(float)));
+    NODE_CHECK(durable_alloc(&T->d_area, size_t(n) * sizeof(float)), "alloc area");
     unsigned long long* d_ties = reinterpret_cast<unsigned long long*>(d_misc + 1);
     leaf_kernel<<<grid_for(nn, kThreads), kThreads, 0, s>>>(nn, n, D, d_level, d_head, d_first, d_lcp, d_leafd,
                                                             codes, perm, T->d_bounds, bound_stride, d_lcnt,
@@ -763,7 +763,7 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     {
         const size_t rec = size_t(nn + h_extra);
         float4* base = nullptr;
-        NODE_CHECK(cudaMalloc(&base, rec * 4 * sizeof(float4)), "alloc nodes");
+        NODE_CHECK(durable_alloc(&base, rec * 4 * sizeof(float4)), "alloc nodes");
         T->nodes.geom = base;
         T->nodes.pm = base + rec;
         T->nodes.nc = base + 2 * rec;
@@ -784,15 +784,15 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
     }
 
     // ---- kept for export, DC and neighbour gathers
-    NODE_CHECK(cudaMalloc(&T->d_node_head, size_t(nn) * 4), "alloc head");
+    NODE_CHECK(durable_alloc(&T->d_node_head, size_t(nn) * 4), "alloc head");
     NODE_CHECK(cudaMemcpyAsync(T->d_node_head, d_head, size_t(nn) * 4, cudaMemcpyDeviceToDevice, s), "copy head");
-    NODE_CHECK(cudaMalloc(&T->d_codes, size_t(n) * 8), "alloc codes");
+    NODE_CHECK(durable_alloc(&T->d_codes, size_t(n) * 8), "alloc codes");
     NODE_CHECK(cudaMemcpyAsync(T->d_codes, codes, size_t(n) * 8, cudaMemcpyDeviceToDevice, s), "copy codes");
-    NODE_CHECK(cudaMalloc(&T->d_perm, size_t(n) * 4), "alloc perm");
+    NODE_CHECK(durable_alloc(&T->d_perm, size_t(n) * 4), "alloc perm");
     NODE_CHECK(cudaMemcpyAsync(T->d_perm, perm, size_t(n) * 4, cudaMemcpyDeviceToDevice, s), "copy perm");
-    NODE_CHECK(cudaMalloc(&T->d_spts, size_t(n) * sizeof(float4)), "alloc spts");
-    NODE_CHECK(cudaMalloc(&T->d_snrm, size_t(n) * sizeof(float4)), "alloc snrm");
-    NODE_CHECK(cudaMalloc(&T->d_wspts, size_t(n) * sizeof(float4)), "alloc wspts");
+    NODE_CHECK(durable_alloc(&T->d_spts, size_t(n) * sizeof(float4)), "alloc spts");
+    NODE_CHECK(durable_alloc(&T->d_snrm, size_t(n) * sizeof(float4)), "alloc snrm");
+    NODE_CHECK(durable_alloc(&T->d_wspts, size_t(n) * sizeof(float4)), "alloc wspts");
     sorted_points_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(n, perm, d_pts, d_nrm, T->origin[0], T->origin[1],
                                                                     T->origin[2], T->d_spts, T->d_snrm, T->d_wspts);
     note_launch();
@@ -803,8 +803,8 @@ int build_tree(mlods_tree_s* T, const float* d_pts, const float* d_nrm, int64_t 
         NODE_CHECK(cudaMemcpy(&root_pm, T->nodes.pm, sizeof root_pm, cudaMemcpyDeviceToHost), "root mass");
         T->root_mass = root_pm.w;
     }
-    cudaFree(nodebuf);
-    cudaFree(bump.base);
+    scratch_free(nodebuf, s);
+    scratch_free(bump.base, s);
 #undef NODE_CHECK
 #undef BUILD_CHECK
     T->device_bytes = int64_t((nn + h_extra) * 4 * sizeof(float4)) + nn * 4 + n * (8 + 4 + 4 + 48) +
@@ -863,7 +863,7 @@ int export_tree(mlods_tree_s* T, int32_t* depth, int32_t* parent, int32_t* first
     std::vector<double> v_mom(nn * 9);
     char* buf = nullptr;
     const size_t bytes = size_t(nn) * (6 * 4 + 6 * 4 + 9 * 8);
-    MLODS_CUDA(cudaMalloc(&buf, bytes));
+    MLODS_CUDA(durable_alloc(&buf, bytes));
     int32_t* d_depth = reinterpret_cast<int32_t*>(buf);
     int32_t* d_parent = d_depth + nn;
     int32_t* d_first = d_parent + nn;
@@ -889,7 +889,7 @@ int export_tree(mlods_tree_s* T, int32_t* depth, int32_t* parent, int32_t* first
     if (e == cudaSuccess) e = cudaMemcpy(v_bmin.data(), d_bmin, nn * 12, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(v_bmax.data(), d_bmax, nn * 12, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(v_mom.data(), d_mom, nn * 72, cudaMemcpyDeviceToHost);
-    cudaFree(buf);
+    durable_free(buf);
     if (e != cudaSuccess) return cuda_fail(e, "export", __FILE__, __LINE__);
     // leaf point lists: single-point leaves hold the point index in `first`,
     // multi-point leaves point at their point records.
