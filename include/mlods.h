@@ -102,7 +102,11 @@ typedef struct mlods_params {
                                  share one walk of the tree (node loads and traversal bookkeeping
                                  paid once); each query's arithmetic is unchanged, only the order
                                  of its float sums differs, so results agree with 1 to float
-                                 rounding.  mlods_tune_schedule picks it by timing. */
+                                 rounding.  mlods_tune_schedule picks it by timing.  Calls of many
+                                 queries (about 350,000 on with 1, 800,000 with 2 or 4, two or more
+                                 iterations, about as many queries as points) walk in packets of
+                                 32 queries whatever the setting; with 1 a query's result does
+                                 not depend on the others there either. */
 } mlods_params;
 
 typedef struct mlods_tree_s* mlods_tree;
@@ -357,8 +361,9 @@ int mlods_last_walk_counts(mlods_tree t, int64_t* lane_visits, int64_t* pruned);
  * [offsets[i], offsets[i+1]), offsets is a HOST array of n_trees + 1 entries
  * starting at 0) onto their trees, writing d_out_pts/d_out_nrm in the same
  * layout.  The launch's warps take a tree's queries one or two at a time from
- * a device counter, the trees with the most work first, and walk them with
- * the tree's own specialisation of the walk (kernel family and terms, blend
+ * a device counter, the trees with the most work first (trees with enough
+ * queries to walk in packets do so in two launches of their own before it),
+ * and walk them with the tree's own specialisation of the walk (kernel family and terms, blend
  * rule, queries per warp), so trees of any size and kernel share the launch.
  * Every tree must be in MLODS_MODE_MLOD with a kernel set; each tree's own
  * cutoff, min_depth, blend rule and convergence mode apply (pruning does not),

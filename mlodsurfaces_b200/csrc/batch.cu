@@ -7,8 +7,9 @@
 // queries two (or one) at a time from a device counter -- the trees with the
 // most work first -- and walk them with the tree's own specialisation of the
 // walk, so trees of very different sizes and kernels load-balance inside a
-// single launch.  A schedule may instead run the largest trees in launches of
-// their own (the single-tree kernel, whose arguments sit in the constant bank)
+// single launch.  Trees with enough queries to walk in packets (project.cuh) do so
+// in launches of their own, and a schedule may run the largest of the others in
+// launches of their own (the single-tree kernel, whose arguments sit in the constant bank)
 // before the shared launch of the rest.  With use_graph the memset / order /
 // kernel sequence is captured once in a CUDA graph and replayed while the
 // buffers, sizes and schedule stay the same.  The autotuner
@@ -38,7 +39,8 @@ struct mlods_batch_s {
     // launch shape (the tuner's pick, or set by the caller)
     mlods_batch_schedule sched{0, 1, 100, mlods::kQueueMostWorkFirst, 0};
     int run_qpw = 1;                  // the walk schedule the launches use
-    std::vector<int> h_solo;          // trees with a launch of their own
+    std::vector<int> h_packet;        // trees whose queries walk in packets
+    std::vector<int> h_solo;          // the others with a launch of their own
     std::vector<mlods::CloudArgs> h_qclouds;  // the other trees: the shared launch's arguments
     std::vector<int64_t> h_qbase, h_qlen;
     int walk_launches = 0;            // launches of the walk per call
@@ -90,20 +92,31 @@ int enqueue(mlods_batch_s* b, const float* d_q, int64_t total, bool timed, cudaS
     }
     const int sm = sm_count_for_current_device();
     if (timed) MLODS_CUDA(cudaEventRecord(b->ev0, s));
-    // the largest trees first, each in a launch of its own: its slice of the
+    // the largest trees first, each in launches of its own: its slice of the
     // batch order, rebased to the tree's own query indices
     unsigned int* solo_counters =
         reinterpret_cast<unsigned int*>(b->d_stats + 8 + queue_groups(int(b->h_qclouds.size())) + 1);
-    for (size_t k = 0; k < b->h_solo.size(); ++k) {
-        const int i = b->h_solo[k];
+    auto solo_args = [&](int i) {
         ProjectArgs pa;
         pa.cloud = b->h_clouds[size_t(i)];
         pa.order = order ? order + b->h_offsets[size_t(i)] : nullptr;
         pa.order_base = order ? uint32_t(b->h_offsets[size_t(i)]) : 0u;
         pa.nq = b->h_offsets[size_t(i) + 1] - b->h_offsets[size_t(i)];
-        pa.counter = solo_counters + k;
+        pa.counter = solo_counters++;
         pa.stats = b->d_stats;
         pa.queries_per_warp = b->run_qpw;
+        return pa;
+    };
+    for (const int i : b->h_packet) {
+        const mlods_tree_s* T = b->trees[size_t(i)];
+        float ext = 0.f;
+        for (int a = 0; a < 3; ++a) ext = std::max(ext, T->BB[a] - T->bb[a]);
+        void* tmp = static_cast<char*>(b->d_order_buf) + up256(size_t(total) * 4);
+        MLODS_CUDA(launch_mlod_packets(solo_args(i), static_cast<uint32_t*>(b->d_order_buf) + b->h_offsets[size_t(i)], tmp,
+                                       ext, sm, s));
+    }
+    for (const int i : b->h_solo) {
+        const ProjectArgs pa = solo_args(i);
         MLODS_CUDA(launch_mlod_project(pa, pa.cloud.kc.type, pa.cloud.rule, sm, s));
     }
     if (!b->h_qclouds.empty()) {
@@ -187,13 +200,15 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
         b->h_offsets.assign(offsets, offsets + n + 1);
     }
     // the trees with a launch of their own (the largest first) and the rest
-    std::vector<int> solo;
+    std::vector<int> packet, solo;
     std::vector<CloudArgs> qclouds;
     std::vector<int64_t> qbase, qlen;
     for (int i = 0; i < n; ++i) {
         const int64_t len = offsets[i + 1] - offsets[i];
         if (len == 0) continue;
-        if (b->sched.solo_min_queries > 0 && len >= b->sched.solo_min_queries) {
+        if (walks_in_packets(clouds[size_t(i)], q, len, b->sched.reorder != 0)) {
+            packet.push_back(i);
+        } else if (b->sched.solo_min_queries > 0 && len >= b->sched.solo_min_queries) {
             solo.push_back(i);
         } else {
             qclouds.push_back(clouds[size_t(i)]);
@@ -201,16 +216,19 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
             qlen.push_back(len);
         }
     }
-    std::stable_sort(solo.begin(), solo.end(), [&](int x, int y) {
+    const auto more_work = [&](int x, int y) {
         return (offsets[x + 1] - offsets[x]) * std::max(clouds[size_t(x)].n_iter, 1) >
                (offsets[y + 1] - offsets[y]) * std::max(clouds[size_t(y)].n_iter, 1);
-    });
-    if (solo != b->h_solo || qbase != b->h_qbase || qlen != b->h_qlen) drop_graph(b);
+    };
+    std::stable_sort(packet.begin(), packet.end(), more_work);
+    std::stable_sort(solo.begin(), solo.end(), more_work);
+    if (packet != b->h_packet || solo != b->h_solo || qbase != b->h_qbase || qlen != b->h_qlen) drop_graph(b);
+    b->h_packet = packet;
     b->h_solo = solo;
     b->h_qclouds = qclouds;
     b->h_qbase = qbase;
     b->h_qlen = qlen;
-    b->walk_launches = int(solo.size()) + (qclouds.empty() ? 0 : queue_groups(int(qclouds.size())));
+    b->walk_launches = 2 * int(packet.size()) + int(solo.size()) + (qclouds.empty() ? 0 : queue_groups(int(qclouds.size())));
     const size_t need = up256(size_t(total) * 4) + query_order_temp_bytes(total);
     if (b->order_bytes < need) {
         drop_graph(b);

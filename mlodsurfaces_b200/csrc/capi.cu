@@ -340,6 +340,7 @@ void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, const float* d_q, floa
     // in place, the buffer must stay in world coordinates for the next call
     c.local_out = (T->params.local_output != 0 && d_out_p != d_q) ? 1 : 0;
     c.qpw = T->params.queries_per_warp;
+    c.n_pts = T->n_pts;
     // kernel-weight pruning: a subtree is dropped below prune_tol times the
     // weight of one average sample sitting at the query (w(0) x mean area)
     c.prune_thr = 0.f;
@@ -475,7 +476,8 @@ size_t project_call_bytes(const mlods_tree_s* T, int64_t n)
 {
     if (T->params.mode != MLODS_MODE_MLOD) return 0;
     const bool reorder = T->params.reorder != 0 && n > 1;
-    return reorder ? al256(size_t(n) * 4) + query_order_temp_bytes(n) : 0;
+    const bool packets = T->params.queries_per_warp == 1 && n >= kPacketMinQueries;  // (they order the queries)
+    return reorder || packets ? al256(size_t(n) * 4) + query_order_temp_bytes(n) : 0;
 }
 
 int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p, float* d_out_n, int iters,
@@ -514,10 +516,10 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
     }
     MLODS_CUDA(cudaMemsetAsync(stats, 0, 8 * sizeof(int64_t), s));
     uint32_t* d_order = nullptr;
+    float ext = 0.f;
+    for (int ax = 0; ax < 3; ++ax) ext = std::max(ext, T->BB[ax] - T->bb[ax]);
     if (reorder) {
         d_order = reinterpret_cast<uint32_t*>(base);
-        float ext = 0.f;
-        for (int a = 0; a < 3; ++a) ext = std::max(ext, T->BB[a] - T->bb[a]);
         MLODS_CUDA(compute_query_order(d_q, n, T->origin, ext, d_order, base + al256(size_t(n) * 4), s));
     }
     const int rule = rule_override >= 0 ? rule_override : T->params.blend_rule;
@@ -528,14 +530,20 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
     a.counter = reinterpret_cast<unsigned int*>(stats + 3);
     a.stats = stats;
     a.queries_per_warp = T->params.queries_per_warp;
+    const int sm = sm_count_for_current_device();
+    const auto launch = [&] {
+        return walks_in_packets(a.cloud, a.queries_per_warp, n, reorder)
+                   ? launch_mlod_packets(a, reinterpret_cast<uint32_t*>(base), base + al256(size_t(n) * 4), ext, sm, s)
+                   : launch_mlod_project(a, T->kc.type, rule, sm, s);
+    };
     if (cs) {
-        MLODS_CUDA(launch_mlod_project(a, T->kc.type, rule, sm_count_for_current_device(), s));
+        MLODS_CUDA(launch());
         return MLODS_OK;
     }
     const int rc = ensure_events(T);
     if (rc != MLODS_OK) return rc;
     MLODS_CUDA(cudaEventRecord(T->ev_start, s));
-    MLODS_CUDA(launch_mlod_project(a, T->kc.type, rule, sm_count_for_current_device(), s));
+    MLODS_CUDA(launch());
     MLODS_CUDA(cudaEventRecord(T->ev_stop, s));
     T->timed = true;
     return MLODS_OK;

@@ -171,6 +171,14 @@ extern "C" int mlods_project_device_noalloc(mlods_tree t, int64_t n, const float
     a.counter = reinterpret_cast<unsigned int*>(stats + 3);
     a.stats = stats;
     a.queries_per_warp = t->params.queries_per_warp;
-    MLODS_CUDA(launch_mlod_project(a, t->kc.type, rule, sm_count_for_current_device(), s));
+    const int sm = sm_count_for_current_device();
+    if (walks_in_packets(a.cloud, a.queries_per_warp, n, t->params.reorder != 0)) {
+        float ext = 0.f;
+        for (int ax = 0; ax < 3; ++ax) ext = std::max(ext, t->BB[ax] - t->bb[ax]);
+        MLODS_CUDA(launch_mlod_packets(a, reinterpret_cast<uint32_t*>(base + kStatsBytes),
+                                       base + kStatsBytes + al256(size_t(n) * 4), ext, sm, s));
+        return MLODS_OK;
+    }
+    MLODS_CUDA(launch_mlod_project(a, t->kc.type, rule, sm, s));
     return MLODS_OK;
 }

@@ -52,6 +52,7 @@ struct CloudArgs {
     float* out_n;
     int local_out;          // 1: out_p holds the result relative to (o0, o1, o2)
     int qpw;                // the tree's walk schedule (queries per warp) for launches of its own
+    int64_t n_pts;          // points of the tree
     float prune_thr;        // > 0: kernel-weight pruning threshold (prune_tol * w(0) * mean sample area)
 };
 
@@ -126,6 +127,35 @@ struct BatchFrame {
     float inv_ext;
     uint32_t rank;
 };
+
+// Whether a projection of n queries runs in packets of 32 (packet.cu).  Where
+// the packets fill the GPU several times over (148 SMs x 28 warps x 32 queries =
+// 133k; the last packets run alone for about 3 ms) and the queries lie about as
+// close as the points, so that neighbours need the same nodes.  Against one
+// query per warp: 350k queries on 350k / 700k points 33.4 / 28.4 ms, not 40.0 /
+// 35.7, 500k rational 8.1, not 14.2, but 150k on 150k 18.1, not 15.6, 200k on
+// 600k 24.9, not 23.9.  Two or four queries per warp already share nodes: 800k on
+// 800k 75.7, not 79.4, 1M-point 51.6, not 59.6, 2M 144, not 172, but 400k on
+// 500k 40.9, not 37.5, and 500k on 2M 48, not 45.  Not with one iteration
+// (walks_wide gives the reason), with pruning, or stopping at a tolerance (a
+// query's end does not fit the state kept between the launches); exact
+// convergence returns the bits of a run without it, which is promised with one
+// query per warp, so there it follows; and so does a call without Morton order
+// (ordered: whether the call asks for it), whose results are promised to be the
+// same: the packets order the queries themselves.  n is the number of queries
+// of the call or request: not what a server cuts from it.
+constexpr int64_t kPacketMinQueries = 350000;
+inline bool walks_in_packets(const CloudArgs& c, int qpw, int64_t n, bool ordered)
+{
+    if (!walks_wide(c) || n >= (int64_t(1) << 32) - 64) return false;
+    if (c.conv_mode != MLODS_CONVERGE_OFF && !(c.conv_mode == MLODS_CONVERGE_EXACT && qpw == 1)) return false;
+    return qpw == 1 ? n >= kPacketMinQueries && 2 * n >= c.n_pts : ordered && n >= 800000 && 4 * n >= 3 * c.n_pts;
+}
+// The whole projection in packets: a's launch arguments; the order of the
+// queries (made here where a.order is null) is rewritten after the first
+// iteration (order: a.nq entries, may be a.order; order_temp: query_order_temp_bytes(a.nq) bytes; extent: the root box's largest).
+cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* order_temp, float extent, int sm_count,
+                                cudaStream_t s);
 
 cudaError_t launch_mlod_project(const ProjectArgs& a, int ktype, int rule, int sm_count, cudaStream_t s);
 

@@ -242,8 +242,10 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
         int n_solo = 0;
         for (size_t i = 0; i < nc && e == cudaSuccess; ++i) {
             const int64_t len = w.h_offsets[i + 1] - w.h_offsets[i];
-            if (len >= solo_min) {
-                // a large piece: the single-tree kernel on its slice of the order
+            // the pieces of a request walk as the whole request would
+            const bool packets = walks_in_packets(w.h_clouds[i], qpw, batch[i].r->n, true);
+            if (packets || len >= solo_min) {
+                // a large piece: launches of its own on its slice of the order
                 ProjectArgs pa;
                 pa.cloud = w.h_clouds[i];
                 pa.order = order + w.h_offsets[i];
@@ -252,7 +254,14 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
                 pa.counter = solo_counters + n_solo++;
                 pa.stats = w.d_stats;
                 pa.queries_per_warp = qpw;
-                e = launch_mlod_project(pa, pa.cloud.kc.type, pa.cloud.rule, sm, w.s);
+                if (packets) {
+                    const mlods_tree_s* T = S->trees[size_t(batch[i].r->tree)];
+                    float ext = 0.f;
+                    for (int a = 0; a < 3; ++a) ext = std::max(ext, T->BB[a] - T->bb[a]);
+                    e = launch_mlod_packets(pa, order + w.h_offsets[i], mem + L.temp, ext, sm, w.s);
+                } else {
+                    e = launch_mlod_project(pa, pa.cloud.kc.type, pa.cloud.rule, sm, w.s);
+                }
             } else {
                 qclouds.push_back(w.h_clouds[i]);
                 qbase.push_back(w.h_offsets[i]);
