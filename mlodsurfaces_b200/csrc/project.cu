@@ -49,15 +49,25 @@ constexpr uint32_t kEntNoBlend = 1u << 31;
 constexpr uint32_t kEntLastOnly = 1u << 30;  // CPU rule multi-point leaf: only the last point is weighted
 
 // Per-warp stack of sibling ranges: h = {first, count | live mask | flags},
-// v[x] = {f, A, dP, g} of query x of the warp; cnt repeats the count word so
-// that the pop scan reads 4 bytes.
+// v[x] = {f, A, dP, g} of query x of the warp.
 template <int CAP, int QPW>
 struct WarpStack {
     uint2 h[CAP];
     float4 v[CAP][QPW];
-    uint32_t cnt[CAP];
 };
 static_assert(sizeof(uint2) * 2 == sizeof(float4), "the stack arrays stay 16-byte aligned for even CAP");
+
+// v + the value o lanes below, where there is one
+__device__ __forceinline__ int add_from_below(int v, int o)
+{
+    int r;
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .s32 t;\n shfl.sync.up.b32 t|p, %1, %2, 0, 0xffffffff;\n"
+        " @p add.s32 t, t, %1;\n @!p mov.s32 t, %1;\n mov.s32 %0, t;\n}"
+        : "=r"(r)
+        : "r"(v), "r"(o));
+    return r;
+}
 
 // Inclusive prefix sum over groups of 16 lanes (4 shuffle steps): exact for
 // lanes 0-15, which are the only ones the pop reads.  A round takes at most
@@ -67,12 +77,8 @@ static_assert(sizeof(uint2) * 2 == sizeof(float4), "the stack arrays stay 16-byt
 // 7.50 ms with two queries per warp).
 __device__ __forceinline__ int warp_incl_scan16(int v)
 {
-    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-        int n = __shfl_up_sync(kFull, v, o);
-        if (lane >= o) v += n;
-    }
+    for (int o = 1; o < 16; o <<= 1) v = add_from_below(v, o);
     return v;
 }
 
@@ -113,7 +119,7 @@ template <int KTYPE, int NSIG, int RULE, int CAP, int QPW, bool PRUNE>
 __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t (&qi)[QPW], int nq,
                                              WarpStack<CAP, QPW>& st, WalkStats& ws)
 {
-    static_assert(QPW >= 1 && QPW <= 4, "one to four queries per warp");
+    static_assert(QPW == 1, "more queries per warp walk packed");
     const bool gpu_rule = RULE < 0 ? c.rule == MLODS_BLEND_GPU : RULE == MLODS_BLEND_GPU;
     const int lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -158,16 +164,14 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
             st.h[0] = make_uint2(0u, w0);
 #pragma unroll
             for (int x = 0; x < QPW; ++x) st.v[0][x] = make_float4(1.f, 0.f, 0.f, 0.f);
-            st.cnt[0] = w0;
         }
         __syncwarp();
         while (top > 0) {
             // ---- pop sibling ranges from the top (at most 16) until 32 lanes are filled
-            int cn = 0;
-            if (lane < top && lane < 16) cn = int(st.cnt[top - 1 - lane] & kEntCount);
+            // (lanes without a range count more than can fit)
+            const int cn = lane < top && lane < 16 ? int(st.h[top - 1 - lane].y & kEntCount) : 0x1000000;
             const int incl = warp_incl_scan16(cn);
-            const uint32_t fit = __ballot_sync(kFull, lane < top && lane < 16 && incl <= 32);
-            const int npop = __popc(fit);
+            const int npop = __popc(__ballot_sync(kFull, incl <= 32));
             const bool partial = npop == 0;  // top range wider than a warp (multi-point leaf)
             const int total = partial ? 32 : __shfl_sync(kFull, incl, npop - 1);
             const uint32_t heads = partial ? 1u : __reduce_or_sync(kFull, lane < npop ? (1u << (incl - cn)) : 0u);
@@ -188,18 +192,12 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
             const int old_top = top;
             if (!partial) top -= npop;
             ws.lane_visits += uint32_t(total);
-            ws.visits += QPW == 1 ? uint32_t(total) : __reduce_add_sync(kFull, active ? uint32_t(__popc(r_live)) : 0u);
             ++ws.rounds;
 
             // ---- evaluate one node per lane, for each of its live queries
-            const uint32_t node = r_first + uint32_t(lane - r_start);
-            float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f), p4 = g4;
-            float4 x4 = make_float4(0.f, 0.f, __uint_as_float(kLeafBit | 1u), 0.f);
-            if (active) {
-                g4 = __ldg(ngeom + node);
-                p4 = __ldg(npm + node);
-                x4 = __ldg(naux + node);
-            }
+            // (lanes past the last range repeat its last node)
+            const uint32_t node = r_first + uint32_t(min(lane - r_start, r_len - 1));
+            const float4 g4 = __ldg(ngeom + node), p4 = __ldg(npm + node), x4 = __ldg(naux + node);
             const float cr = cutoff * g4.w;
             const bool blend = active && !(r_cnt & kEntNoBlend);
             const int seg_end = r_start + r_len;
@@ -232,21 +230,20 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
             const uint32_t info = __float_as_uint(x4.z);
             const uint32_t nfirst = __float_as_uint(x4.y);
             const bool leaf = (info & kLeafBit) != 0;
-            const bool multi = (info & kMultiBit) != 0;
             const uint32_t cnt = node_count(info);
             // opened for every live query whatever its distance: the points of
             // a multi-point leaf, the children of a node above min_depth
-            const bool opens_all = leaf ? multi : node_depth(info) < min_depth;
-            uint32_t term = 0, near = 0;
-            if (active && !opens_all) {
+            const bool opens_all = leaf ? (info & kMultiBit) != 0 : node_depth(info) < min_depth;
+            // the distance beyond which the node ends a walk (a query that is
+            // NaN is beyond any: it fails with its sums)
+            const float thr = opens_all ? INFINITY : (leaf ? -1.f : cr);
+            const uint32_t on = active ? r_live : 0u;
+            uint32_t far = 0;
 #pragma unroll
-                for (int x = 0; x < QPW; ++x) {
-                    if (!((r_live >> x) & 1u)) continue;
-                    if (leaf || dist[x] > cr) term |= 1u << x;
-                    else near |= 1u << x;
-                }
-            }
-            if (PRUNE && near) {
+            for (int x = 0; x < QPW; ++x)
+                if (!(dist[x] <= thr)) far |= 1u << x;
+            uint32_t term = on & far, near = on & ~far;
+            if (PRUNE && near && !opens_all) {
                 // kernel-weight pruning (extension, off by default): a near
                 // node whose whole subtree can weigh no more than the
                 // threshold -- the kernel decreases with distance, so w at
@@ -264,10 +261,7 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
                     }
                 }
             }
-            const uint32_t child_live = active ? (opens_all ? r_live : near) : 0u;
-            const bool push = child_live != 0;
-            const uint32_t p_cnt = cnt | (child_live << kEntLiveShift) |
-                                   (opens_all ? (kEntNoBlend | (leaf && !gpu_rule ? kEntLastOnly : 0u)) : 0u);
+            const bool push = near != 0;
 
             float4 n4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (term) n4 = __ldg(nnc + node);
@@ -301,7 +295,6 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
                 rest.x += 32u;
                 rest.y -= 32u;
                 st.h[old_top - 1] = rest;
-                st.cnt[old_top - 1] = rest.y;
             }
             const uint32_t pm = __ballot_sync(kFull, push);
             const int npush = __popc(pm);
@@ -310,10 +303,10 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
             } else {
                 if (push) {
                     const int pos = top + __popc(pm & lt_mask);
-                    st.h[pos] = make_uint2(nfirst, p_cnt);
+                    st.h[pos] = make_uint2(nfirst, cnt | (near << kEntLiveShift) |
+                                                       (opens_all ? (kEntNoBlend | (leaf && !gpu_rule ? kEntLastOnly : 0u)) : 0u));
 #pragma unroll
                     for (int x = 0; x < QPW; ++x) st.v[pos][x] = make_float4(f[x], A[x], pv_dP[x], pv_g[x]);
-                    st.cnt[pos] = p_cnt;
                 }
                 top += npush;
             }
@@ -356,6 +349,7 @@ __device__ __forceinline__ void project_walk(const CloudArgs& c, const uint32_t 
         live &= ~__ballot_sync(kFull, mine && stop);
     }
     failed = __reduce_or_sync(kFull, failed);
+    ws.visits = ws.lane_visits;  // one query: it needs every node
     if (lane < nq) {
         float* op = c.out_p + 3 * int64_t(my_q);
         float* on = c.out_n + 3 * int64_t(my_q);
@@ -443,6 +437,7 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
     float nrm[3] = {0.f, 0.f, 0.f};
     uint32_t live = (1u << nq) - 1u;  // queries still iterating (warp-uniform)
     uint32_t failed = 0;
+    uint32_t my_visits = 0;
     for (int it = 0; it < c.n_iter && live; ++it) {
         // queries 2j and 2j + 1 form pair j
         float2 qx[NP], qy[NP], qz[NP];
@@ -469,16 +464,14 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
                 st.v[0][2 * j] = make_float4(1.f, 1.f, 0.f, 0.f);  // f f A A
                 st.v[0][2 * j + 1] = make_float4(0.f, 0.f, 0.f, 0.f);  // dP dP g g
             }
-            st.cnt[0] = w0;
         }
         __syncwarp();
         while (top > 0) {
             // ---- pop sibling ranges from the top (at most 16) until 32 lanes are filled
-            int cn = 0;
-            if (lane < top && lane < 16) cn = int(st.cnt[top - 1 - lane] & kEntCount);
+            // (lanes without a range count more than can fit)
+            const int cn = lane < top && lane < 16 ? int(st.h[top - 1 - lane].y & kEntCount) : 0x1000000;
             const int incl = warp_incl_scan16(cn);
-            const uint32_t fit = __ballot_sync(kFull, lane < top && lane < 16 && incl <= 32);
-            const int npop = __popc(fit);
+            const int npop = __popc(__ballot_sync(kFull, incl <= 32));
             const bool partial = npop == 0;  // top range wider than a warp (multi-point leaf)
             const int total = partial ? 32 : __shfl_sync(kFull, incl, npop - 1);
             const uint32_t heads = partial ? 1u : __reduce_or_sync(kFull, lane < npop ? (1u << (incl - cn)) : 0u);
@@ -500,23 +493,18 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
             const int old_top = top;
             if (!partial) top -= npop;
             ws.lane_visits += uint32_t(total);
-            ws.visits += __reduce_add_sync(kFull, active ? uint32_t(__popc(r_live)) : 0u);
+            my_visits += active ? uint32_t(__popc(r_live)) : 0u;
             ++ws.rounds;
 
             // ---- evaluate one node per lane, for every query at once
-            const uint32_t node = r_first + uint32_t(lane - r_start);
-            float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f), p4 = g4;
-            float4 x4 = make_float4(0.f, 0.f, __uint_as_float(kLeafBit | 1u), 0.f);
+            // (lanes past the last range repeat its last node)
+            const uint32_t node = r_first + uint32_t(min(lane - r_start, r_len - 1));
+            const float4 g4 = __ldg(ngeom + node), p4 = __ldg(npm + node), x4 = __ldg(naux + node);
             // the normal record is needed only where the node ends a walk;
             // loading it with the others hides its latency, which measured
             // faster in the single-tree kernel and slower in the queue kernel
-            float4 n4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (active) {
-                g4 = __ldg(ngeom + node);
-                p4 = __ldg(npm + node);
-                x4 = __ldg(naux + node);
-                if (EARLY_NC) n4 = __ldg(nnc + node);
-            }
+            float4 n4;
+            if (EARLY_NC) n4 = __ldg(nnc + node);
             const float cr = cutoff * g4.w;
             const bool blend = active && !(r_cnt & kEntNoBlend);
             const int seg_end = r_start + r_len;
@@ -533,7 +521,7 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
                     const float2 dC = make_float2(fmaxf(dCs.x, 0.f), fmaxf(dCs.y, 0.f));
                     const float2 dP = make_float2(VB[j].x, VB[j].y);
                     const float2 den = add2(dP, dC);
-                    const float2 t = mul2(dP, make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y)));
+                    const float2 t = mul2(dP, make_float2(rcp_fast(den.x), rcp_fast(den.y)));
                     const float2 a = mul2(splat2(kPiRef), t);
                     beta = fma2(splat2(-0.5f), make_float2(__cosf(a.x), __cosf(a.y)), splat2(0.5f));
                     kcon = mul2(sub2(splat2(1.f), beta), make_float2(VB[j].z, VB[j].w));
@@ -567,22 +555,20 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
             const uint32_t info = __float_as_uint(x4.z);
             const uint32_t nfirst = __float_as_uint(x4.y);
             const bool leaf = (info & kLeafBit) != 0;
-            const bool multi = (info & kMultiBit) != 0;
             const uint32_t cnt = node_count(info);
             // opened for every live query whatever its distance: the points of
             // a multi-point leaf, the children of a node above min_depth
-            const bool opens_all = leaf ? multi : node_depth(info) < min_depth;
-            uint32_t term = 0, near = 0;
-            if (active && !opens_all) {
+            const bool opens_all = leaf ? (info & kMultiBit) != 0 : node_depth(info) < min_depth;
+            // the distance beyond which the node ends a walk (a query that is
+            // NaN is beyond any: it fails with its sums)
+            const float thr = opens_all ? INFINITY : (leaf ? -1.f : cr);
+            const uint32_t on = active ? r_live : 0u;
+            uint32_t far = 0;
 #pragma unroll
-                for (int x = 0; x < QPW; ++x) {
-                    if (!((r_live >> x) & 1u)) continue;
-                    const float d = (x & 1) ? dist[x >> 1].y : dist[x >> 1].x;
-                    if (leaf || d > cr) term |= 1u << x;
-                    else near |= 1u << x;
-                }
-            }
-            if (PRUNE && near) {
+            for (int x = 0; x < QPW; ++x)
+                if (!(((x & 1) ? dist[x >> 1].y : dist[x >> 1].x) <= thr)) far |= 1u << x;
+            uint32_t term = on & far, near = on & ~far;
+            if (PRUNE && near && !opens_all) {
                 // kernel-weight pruning (extension, off by default), as in the
                 // general walk
 #pragma unroll
@@ -599,12 +585,9 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
                     }
                 }
             }
-            const uint32_t child_live = active ? (opens_all ? r_live : near) : 0u;
-            const bool push = child_live != 0;
-            const uint32_t p_cnt = cnt | (child_live << kEntLiveShift) |
-                                   (opens_all ? (kEntNoBlend | (leaf && !gpu_rule ? kEntLastOnly : 0u)) : 0u);
+            const bool push = near != 0;
 
-            const float inv_m = __fdividef(1.f, gpu_rule ? p4.w : float(cnt));
+            const float inv_m = rcp_fast(gpu_rule ? p4.w : float(cnt));
             if (!EARLY_NC && term) n4 = __ldg(nnc + node);
             float2 pv_dP[NP], pv_g[NP];
 #pragma unroll
@@ -642,7 +625,6 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
                 rest.x += 32u;
                 rest.y -= 32u;
                 st.h[old_top - 1] = rest;
-                st.cnt[old_top - 1] = rest.y;
             }
             const uint32_t pmask = __ballot_sync(kFull, push);
             const int npush = __popc(pmask);
@@ -651,13 +633,13 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
             } else {
                 if (push) {
                     const int pos = top + __popc(pmask & lt_mask);
-                    st.h[pos] = make_uint2(nfirst, p_cnt);
+                    st.h[pos] = make_uint2(nfirst, cnt | (near << kEntLiveShift) |
+                                                       (opens_all ? (kEntNoBlend | (leaf && !gpu_rule ? kEntLastOnly : 0u)) : 0u));
 #pragma unroll
                     for (int j = 0; j < NP; ++j) {
                         st.v[pos][2 * j] = make_float4(f[j].x, f[j].y, A[j].x, A[j].y);
                         st.v[pos][2 * j + 1] = make_float4(pv_dP[j].x, pv_dP[j].y, pv_g[j].x, pv_g[j].y);
                     }
-                    st.cnt[pos] = p_cnt;
                 }
                 top += npush;
             }
@@ -700,6 +682,7 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
         live &= ~__ballot_sync(kFull, mine && stop);
     }
     failed = __reduce_or_sync(kFull, failed);
+    ws.visits = __reduce_add_sync(kFull, my_visits);
     if (lane < nq) {
         float* op = c.out_p + 3 * int64_t(my_q);
         float* on = c.out_n + 3 * int64_t(my_q);
@@ -746,17 +729,6 @@ struct WideLimit {
     static_assert(kPop > 32, "stack too small for a full round");
 };
 
-// v + the value o lanes below, where there is one
-__device__ __forceinline__ int add_from_below(int v, int o)
-{
-    int r;
-    asm volatile(
-        "{\n .reg .pred p;\n .reg .s32 t;\n shfl.sync.up.b32 t|p, %1, %2, 0, 0xffffffff;\n"
-        " @p add.s32 t, t, %1;\n @!p mov.s32 t, %1;\n mov.s32 %0, t;\n}"
-        : "=r"(r)
-        : "r"(v), "r"(o));
-    return r;
-}
 template <int KTYPE, int NSIG, int RULE, int CAP>
 __device__ __forceinline__ void project_wide(const CloudArgs& c, uint32_t my_q, WideStack<CAP>& st, WalkStats& ws)
 {

@@ -25,7 +25,7 @@ namespace mlods
 #endif
 constexpr int kProjectThreads = 128;                          // 4 warps per block, one walk per warp at a time
 constexpr int kProjectMinBlocks = MLODS_PROJECT_MIN_BLOCKS;  // 10 -> 40 warps per SM, <= 48 registers
-constexpr int kProjectStackCap = MLODS_PROJECT_STACK_CAP;    // sibling ranges per warp (28 bytes each)
+constexpr int kProjectStackCap = MLODS_PROJECT_STACK_CAP;    // sibling ranges per warp (24 bytes each)
 // the paired walk (two queries per warp): more registers and a wider stack entry
 constexpr int kProjectPairMinBlocks = MLODS_PROJECT_PAIR_MIN_BLOCKS;
 constexpr int kProjectPairStackCap = MLODS_PROJECT_PAIR_STACK_CAP;
