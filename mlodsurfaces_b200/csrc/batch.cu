@@ -232,10 +232,10 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
     const size_t need = up256(size_t(total) * 4) + query_order_temp_bytes(total);
     if (b->order_bytes < need) {
         drop_graph(b);
-        cudaFree(b->d_order_buf);
+        durable_free(b->d_order_buf);
         b->d_order_buf = nullptr;
         b->order_bytes = 0;
-        MLODS_CUDA(cudaMalloc(&b->d_order_buf, need));
+        MLODS_CUDA(durable_alloc(&b->d_order_buf, need));
         b->order_bytes = need;
     }
     *total_out = total;
@@ -325,9 +325,9 @@ int mlods_batch_create(const mlods_tree* trees, int32_t n_trees, mlods_batch* ou
     const size_t n_groups = size_t(queue_groups(n_trees)) + 1;
     b->stats_bytes = (8 * sizeof(int64_t) + n_groups * sizeof(uint64_t) + size_t(n_trees) * sizeof(unsigned int) +
                       255) / 256 * 256;
-    cudaError_t e = cudaMalloc(&b->d_offsets, size_t(n_trees + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_frames, size_t(n_trees) * sizeof(BatchFrame));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_stats, b->stats_bytes);
+    cudaError_t e = durable_alloc(&b->d_offsets, size_t(n_trees + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = durable_alloc(&b->d_frames, size_t(n_trees) * sizeof(BatchFrame));
+    if (e == cudaSuccess) e = durable_alloc(&b->d_stats, b->stats_bytes);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
     if (e != cudaSuccess) {
@@ -343,10 +343,10 @@ int mlods_batch_free(mlods_batch b)
     if (!b) return MLODS_OK;
     DeviceGuard guard(b->device);
     drop_graph(b);
-    cudaFree(b->d_offsets);
-    cudaFree(b->d_frames);
-    cudaFree(b->d_stats);
-    cudaFree(b->d_order_buf);
+    durable_free(b->d_offsets);
+    durable_free(b->d_frames);
+    durable_free(b->d_stats);
+    durable_free(b->d_order_buf);
     if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);

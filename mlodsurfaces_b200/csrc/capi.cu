@@ -760,8 +760,8 @@ int mlods_queries_free(mlods_queries q)
         set_last_error("null query buffer");
         return MLODS_ERR_INVALID;
     }
-    cudaFree(q->d_q);
-    cudaFree(q->d_qn);
+    durable_free(q->d_q);
+    durable_free(q->d_qn);
     q->d_q = q->d_qn = nullptr;
     q->n = q->cap = 0;
     return MLODS_OK;
@@ -784,8 +784,8 @@ int mlods_queries_upload(mlods_queries q, int64_t n, const float* pts, void* str
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (q->cap < n) {
         mlods_queries_free(q);
-        MLODS_CUDA(cudaMalloc(&q->d_q, size_t(n) * 3 * sizeof(float)));
-        MLODS_CUDA(cudaMalloc(&q->d_qn, size_t(n) * 3 * sizeof(float)));
+        MLODS_CUDA(durable_alloc(&q->d_q, size_t(n) * 3 * sizeof(float)));
+        MLODS_CUDA(durable_alloc(&q->d_qn, size_t(n) * 3 * sizeof(float)));
         q->cap = n;
     }
     q->n = n;
@@ -841,11 +841,11 @@ int mlods_queries_reorganize(mlods_queries q, int64_t n_invalid, const uint32_t*
         }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint32_t* d_inv = nullptr;
-    MLODS_CUDA(cudaMalloc(&d_inv, size_t(n_invalid) * 4));
+    MLODS_CUDA(durable_alloc(&d_inv, size_t(n_invalid) * 4));
     cudaError_t e = cudaMemcpyAsync(d_inv, invalid, size_t(n_invalid) * 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = launch_reorganize(q->d_q, d_inv, n_invalid, end_valid, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_inv);
+    durable_free(d_inv);
     if (e != cudaSuccess) return cuda_fail(e, "queries_reorganize", __FILE__, __LINE__);
     return MLODS_OK;
 }
@@ -1016,7 +1016,7 @@ int mlods_knn_host(mlods_tree t, int64_t n, const float* q, int32_t k, int32_t* 
     }
     char* d = nullptr;
     const size_t qb = size_t(n) * 12, ib = size_t(n) * size_t(k) * 4;
-    MLODS_CUDA(cudaMalloc(&d, qb + 2 * ib));
+    MLODS_CUDA(durable_alloc(&d, qb + 2 * ib));
     float* d_q = reinterpret_cast<float*>(d);
     int32_t* d_idx = reinterpret_cast<int32_t*>(d + qb);
     float* d_d2 = reinterpret_cast<float*>(d + qb + ib);
@@ -1025,7 +1025,7 @@ int mlods_knn_host(mlods_tree t, int64_t n, const float* q, int32_t k, int32_t* 
     if (e == cudaSuccess) rc = mlods_knn(t, n, d_q, k, d_idx, d_d2, nullptr);
     if (e == cudaSuccess && rc == MLODS_OK) e = cudaMemcpy(idx, d_idx, ib, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && rc == MLODS_OK) e = cudaMemcpy(d2, d_d2, ib, cudaMemcpyDeviceToHost);
-    cudaFree(d);
+    durable_free(d);
     if (rc != MLODS_OK) return rc;
     if (e != cudaSuccess) return cuda_fail(e, "knn host", __FILE__, __LINE__);
     return MLODS_OK;

@@ -435,9 +435,9 @@ int mesh_project(mlods_tree_s* T, mlods_mesh_s* m, int iters, cudaStream_t s)
     const int64_t nv = int64_t(m->pos.size() / 3);
     if (nv == 0) return MLODS_OK;
     float* d = nullptr;
-    MLODS_CUDA(cudaMalloc(&d, size_t(nv) * 36));
+    MLODS_CUDA(durable_alloc(&d, size_t(nv) * 36));
     auto done = [&](int rc) {
-        cudaFree(d);
+        durable_free(d);
         return rc;
     };
     cudaError_t e = cudaMemcpyAsync(d, m->pos.data(), size_t(nv) * 12, cudaMemcpyHostToDevice, s);
