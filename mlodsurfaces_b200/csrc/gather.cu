@@ -18,6 +18,7 @@
 
 #include "gather.cuh"
 #include "tree.cuh"
+#include "walk.cuh"
 
 namespace mlods
 {
@@ -48,6 +49,9 @@ static_assert(kBatchPopLimit > 0, "gather stack too small for a depth-first walk
 struct GStack {
     uint32_t first[kGatherCap];
     uint32_t cnt[kGatherCap];
+    // neighbour searches: candidates waiting to be merged, up to 31 and a round's
+    float cand_d[64];
+    uint32_t cand_o[64], cand_p[64];
 };
 
 // Per-warp state of a kNN projection query between iterations (uniform over
@@ -73,27 +77,29 @@ __device__ __forceinline__ bool key_less(float da, uint32_t oa, float db, uint32
     return da < db || (da == db && oa < ob);
 }
 
+// One compare-exchange of a bitonic network over the lanes: the lane keeps the
+// smaller of its own and lane ^ j's (d, o, p) if want_min, else the larger.
+__device__ __forceinline__ void warp_exchange(float& d, uint32_t& o, uint32_t& p, int j, bool want_min)
+{
+    const float od = __shfl_xor_sync(kFull, d, j);
+    const uint32_t oo = __shfl_xor_sync(kFull, o, j);
+    const uint32_t op = __shfl_xor_sync(kFull, p, j);
+    if (key_less(od, oo, d, o) == want_min) {
+        d = od;
+        o = oo;
+        p = op;
+    }
+}
+
 // Bitonic sort of one (d, o, p) per lane; ascending unless `desc`.
 __device__ __forceinline__ void warp_sort(float& d, uint32_t& o, uint32_t& p, bool desc)
 {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1) {
+        const bool up = ((lane & k) == 0) != desc;
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const float od = __shfl_xor_sync(kFull, d, j);
-            const uint32_t oo = __shfl_xor_sync(kFull, o, j);
-            const uint32_t op = __shfl_xor_sync(kFull, p, j);
-            const bool up = (((lane & k) == 0) != desc);
-            const bool lower = (lane & j) == 0;
-            const bool other_less = key_less(od, oo, d, o);
-            const bool take = (lower == up) ? other_less : (!other_less && (od != d || oo != o));
-            if (take) {
-                d = od;
-                o = oo;
-                p = op;
-            }
-        }
+        for (int j = k >> 1; j > 0; j >>= 1) warp_exchange(d, o, p, j, ((lane & j) == 0) == up);
     }
 }
 
@@ -114,18 +120,7 @@ __device__ __forceinline__ void warp_merge(float& d, uint32_t& o, uint32_t& p, f
         lost = cd;
     }
 #pragma unroll
-    for (int j = 16; j > 0; j >>= 1) {
-        const float od = __shfl_xor_sync(kFull, d, j);
-        const uint32_t oo = __shfl_xor_sync(kFull, o, j);
-        const uint32_t op = __shfl_xor_sync(kFull, p, j);
-        const bool lower = (lane & j) == 0;
-        const bool other_less = key_less(od, oo, d, o);
-        if (lower ? other_less : (!other_less && (od != d || oo != o))) {
-            d = od;
-            o = oo;
-            p = op;
-        }
-    }
+    for (int j = 16; j > 0; j >>= 1) warp_exchange(d, o, p, j, (lane & j) == 0);
 }
 
 __device__ __forceinline__ float warp_sum_f(float v)
@@ -149,41 +144,28 @@ __device__ __forceinline__ float warp_min_f(float v)
     return v;
 }
 
-__device__ __forceinline__ int warp_incl_scan_i(int v)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int n = __shfl_up_sync(kFull, v, o);
-        if (lane >= o) v += n;
-    }
-    return v;
-}
-
 // Morton code of a world point on the tree's split lattice (the descent of
-// the build, with the split recomputed from the float bound table).
+// the build, with the split recomputed from the float bound table).  Lane a < 3
+// descends axis a, a chain of max_depth dependent loads; lane d then places
+// level d's bits.
 __device__ uint64_t lattice_code(const GatherArgs& a, float wx, float wy, float wz)
 {
-    const float w[3] = {wx, wy, wz};
-    uint32_t cell[3];
-    for (int ax = 0; ax < 3; ++ax) {
-        const float* B = a.bounds + ax * a.bounds_stride;
-        const double x = double(w[ax]);
-        uint32_t k = 0;
-        for (int d = 0; d < a.max_depth; ++d) {
-            const int64_t off = ((int64_t(1) << d) - 1) + d;
-            const double s = (double(__ldg(B + off + k)) + double(__ldg(B + off + k + 1))) / 2.0;
-            k = 2u * k + (x > s ? 1u : 0u);
-        }
-        cell[ax] = k;
-    }
-    uint64_t code = 0;
+    const int lane = threadIdx.x & 31;
+    const int ax = lane < 3 ? lane : 0;
+    const float* B = a.bounds + ax * a.bounds_stride;
+    const double x = double(ax == 0 ? wx : (ax == 1 ? wy : wz));
+    uint32_t k = 0;
     for (int d = 0; d < a.max_depth; ++d) {
-        const int b = a.max_depth - 1 - d;
-        const uint64_t g = ((cell[0] >> b) & 1u) | (((cell[1] >> b) & 1u) << 1) | (((cell[2] >> b) & 1u) << 2);
-        code |= g << (3 * b);
+        const int64_t off = ((int64_t(1) << d) - 1) + d;
+        const double s = (double(__ldg(B + off + k)) + double(__ldg(B + off + k + 1))) / 2.0;
+        k = 2u * k + (x > s ? 1u : 0u);
     }
-    return code;
+    const uint32_t cx = __shfl_sync(kFull, k, 0), cy = __shfl_sync(kFull, k, 1), cz = __shfl_sync(kFull, k, 2);
+    uint64_t code = 0;
+    if (lane < a.max_depth)
+        code = uint64_t(((cx >> lane) & 1u) | (((cy >> lane) & 1u) << 1) | (((cz >> lane) & 1u) << 2)) << (3 * lane);
+    const uint32_t lo = __reduce_or_sync(kFull, uint32_t(code)), hi = __reduce_or_sync(kFull, uint32_t(code >> 32));
+    return (uint64_t(hi) << 32) | lo;
 }
 
 // First sorted position whose code is > qcode, found with 32-way splits.
@@ -300,7 +282,7 @@ __global__ void __launch_bounds__(kGatherThreads, MODE == 0 ? kKnnMinBlocks : kG
             // the (k+1)-th distance, so that the search also bounds the points
             // it leaves out; for the kNN sets the k-th
             float bound = INFINITY;
-            bool search = true;
+            bool search = true, unsorted = false, window = false;
             float warm = INFINITY;  // kNN projection, iteration > 0: the search's starting bound
             if (MODE == 0 && it > 0) {
                 const double ddx = double(wx) - double(carry.px), ddy = double(wy) - double(carry.py),
@@ -329,8 +311,7 @@ __global__ void __launch_bounds__(kGatherThreads, MODE == 0 ? kKnnMinBlocks : kG
                         // after a short step they are mostly still in order
                         const float dn = __shfl_down_sync(kFull, best_d, 1);
                         const uint32_t on = __shfl_down_sync(kFull, best_o, 1);
-                        if (__any_sync(kFull, lane < k - 1 && key_less(dn, on, best_d, best_o)))
-                            warp_sort(best_d, best_o, best_p, false);
+                        unsorted = __any_sync(kFull, lane < k - 1 && key_less(dn, on, best_d, best_o));
                         if (lane == 0) {
                             carry.out_lo = out_lo - step;
                             carry.out_hi = out_hi + step;
@@ -370,20 +351,39 @@ __global__ void __launch_bounds__(kGatherThreads, MODE == 0 ? kKnnMinBlocks : kG
                         best_o = __float_as_uint(p.w);
                         best_p = uint32_t(j);
                     }
-                    warp_sort(best_d, best_o, best_p, false);
-                    if (MODE == 0 && k == 32) {
-                        // a 33rd point beside the window bounds the 33rd distance
-                        const int64_t xp = w1 < a.n_pts ? w1 : w0 - 1;
-                        const float xd2 = xp >= 0 ? kd_dist2(__ldg(a.wspts + xp), wx, wy, wz) : INFINITY;
-                        bound = fmaxf(__shfl_sync(kFull, best_d, 31), xd2);
-                    } else {
-                        bound = __shfl_sync(kFull, best_d, MODE == 0 ? k : k - 1);
-                    }
+                    unsorted = window = true;
                 } else {
                     bound = float(r2ball) * (1.f + 1e-6f);
                 }
             }
+            // (one instance of the sort for the window and the kept points, and
+            // below one of the merge: the kernel's code has to stay in the
+            // instruction cache, a sixth of its stalls)
+            if (MODE != 1 && unsorted) warp_sort(best_d, best_o, best_p, false);
+            if (MODE != 1 && window) {
+                if (MODE == 0 && k == 32) {
+                    // a 33rd point beside the window bounds the 33rd distance
+                    const int64_t xp = w1 < a.n_pts ? w1 : w0 - 1;
+                    const float xd2 = xp >= 0 ? kd_dist2(__ldg(a.wspts + xp), wx, wy, wz) : INFINITY;
+                    bound = fmaxf(__shfl_sync(kFull, best_d, 31), xd2);
+                } else {
+                    bound = __shfl_sync(kFull, best_d, MODE == 0 ? k : k - 1);
+                }
+            }
             // ---- octree walk
+            int waiting = 0;  // candidates in the buffer
+            // merges the first n of them into the best list and tightens the
+            // bound: the (k+1)-th (kNN projection) or k-th distance so far
+            auto merge_waiting = [&](int n) {
+                const bool have = lane < n;
+                float lost = INFINITY;
+                warp_merge(best_d, best_o, best_p, have ? st.cand_d[lane] : INFINITY, have ? st.cand_o[lane] : 0xFFFFFFFFu,
+                           have ? st.cand_p[lane] : 0xFFFFFFFFu, lost);
+                if (MODE == 0 && k == 32)
+                    bound = fminf(bound, warp_min_f(lost));
+                else
+                    bound = fminf(bound, __shfl_sync(kFull, best_d, MODE == 0 ? k : k - 1));
+            };
             int top = search ? 1 : 0;
             if (lane == 0 && search) {
                 st.first[0] = 0;
@@ -391,37 +391,27 @@ __global__ void __launch_bounds__(kGatherThreads, MODE == 0 ? kKnnMinBlocks : kG
             }
             __syncwarp();
             while (top > 0) {
-                uint32_t e_first = 0, e_cnt = 0;
-                int c = 0;
-                if (lane < top) {
-                    e_first = st.first[top - 1 - lane];
-                    e_cnt = st.cnt[top - 1 - lane];
-                    c = int(e_cnt & kGCount);
-                }
-                const int incl = warp_incl_scan_i(c);
                 const int pop_lanes = top > kBatchPopLimit ? 1 : top;  // depth-first near the cap
-                const uint32_t fit = __ballot_sync(kFull, lane < pop_lanes && incl <= 32);
-                int npop = __popc(fit);
+                // (lanes without a range count more than can fit)
+                const int c = lane < pop_lanes ? int(st.cnt[top - 1 - lane] & kGCount) : 0x1000000;
+                int incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) incl = add_from_below(incl, o);
+                const int npop = __popc(__ballot_sync(kFull, incl <= 32));
                 const bool partial = npop == 0;
-                int total;
-                uint32_t headbit;
-                if (partial) {
-                    total = 32;
-                    headbit = lane == 0 ? 1u : 0u;
-                } else {
-                    total = __shfl_sync(kFull, incl, npop - 1);
-                    headbit = lane < npop ? (1u << (incl - c)) : 0u;
-                }
-                const uint32_t heads = __reduce_or_sync(kFull, headbit);
+                const int total = partial ? 32 : __shfl_sync(kFull, incl, npop - 1);
+                const uint32_t heads = partial ? 1u : __reduce_or_sync(kFull, lane < npop ? 1u << (incl - c) : 0u);
                 const bool active = lane < total;
-                const int e = active ? __popc(heads & (lane == 31 ? kFull : ((2u << lane) - 1u))) - 1 : 0;
-                const uint32_t r_first = __shfl_sync(kFull, e_first, e);
-                const uint32_t r_cnt = __shfl_sync(kFull, e_cnt, e);
-                const int r_start = partial ? 0 : __shfl_sync(kFull, incl - c, e);
+                // entry of this lane: the range that starts at the highest head
+                // bit at or below it
+                const uint32_t hb = heads & (lane == 31 ? kFull : ((2u << lane) - 1u));
+                const int r_start = 31 - __clz(hb);
+                const uint32_t r_first = st.first[top - __popc(hb)], r_cnt = st.cnt[top - __popc(hb)];
                 if (partial) {
+                    __syncwarp();
                     if (lane == 0) {
-                        st.first[top - 1] = e_first + 32u;
-                        st.cnt[top - 1] = e_cnt - 32u;
+                        st.first[top - 1] = r_first + 32u;
+                        st.cnt[top - 1] = r_cnt - 32u;
                     }
                 } else {
                     top -= npop;
@@ -490,15 +480,16 @@ __global__ void __launch_bounds__(kGatherThreads, MODE == 0 ? kKnnMinBlocks : kG
                     }
                 }
                 if (MODE != 1) {
-                    if (__any_sync(kFull, cd <= bound && cd < INFINITY)) {
-                        float lost = INFINITY;
-                        warp_merge(best_d, best_o, best_p, cd, co, cp, lost);
-                        // the (k+1)-th (kNN projection) or k-th distance so far
-                        if (MODE == 0 && k == 32)
-                            bound = fminf(bound, warp_min_f(lost));
-                        else
-                            bound = fminf(bound, __shfl_sync(kFull, best_d, MODE == 0 ? k : k - 1));
+                    // wait for a warp of candidates before a merge
+                    const bool take = cd <= bound && cd < INFINITY;
+                    const uint32_t tm = __ballot_sync(kFull, take);
+                    if (take) {
+                        const int at = waiting + __popc(tm & lt_mask);
+                        st.cand_d[at] = cd;
+                        st.cand_o[at] = co;
+                        st.cand_p[at] = cp;
                     }
+                    waiting += __popc(tm);
                 }
                 const uint32_t pm = __ballot_sync(kFull, push);
                 const int npush = __popc(pm);
@@ -513,6 +504,25 @@ __global__ void __launch_bounds__(kGatherThreads, MODE == 0 ? kKnnMinBlocks : kG
                     top += npush;
                 }
                 __syncwarp();
+                while (MODE != 1 && (waiting >= 32 || (top == 0 && waiting > 0))) {
+                    merge_waiting(waiting);
+                    const int rest = waiting - 32;
+                    float md = 0.f;
+                    uint32_t mo = 0, mp = 0;
+                    if (lane < rest) {
+                        md = st.cand_d[32 + lane];
+                        mo = st.cand_o[32 + lane];
+                        mp = st.cand_p[32 + lane];
+                    }
+                    __syncwarp();
+                    if (lane < rest) {
+                        st.cand_d[lane] = md;
+                        st.cand_o[lane] = mo;
+                        st.cand_p[lane] = mp;
+                    }
+                    __syncwarp();
+                    waiting = max(rest, 0);
+                }
             }
             if (overflow) {
                 failed = true;

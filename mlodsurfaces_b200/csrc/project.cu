@@ -57,18 +57,6 @@ struct WarpStack {
 };
 static_assert(sizeof(uint2) * 2 == sizeof(float4), "the stack arrays stay 16-byte aligned for even CAP");
 
-// v + the value o lanes below, where there is one
-__device__ __forceinline__ int add_from_below(int v, int o)
-{
-    int r;
-    asm volatile(
-        "{\n .reg .pred p;\n .reg .s32 t;\n shfl.sync.up.b32 t|p, %1, %2, 0, 0xffffffff;\n"
-        " @p add.s32 t, t, %1;\n @!p mov.s32 t, %1;\n mov.s32 %0, t;\n}"
-        : "=r"(r)
-        : "r"(v), "r"(o));
-    return r;
-}
-
 // Inclusive prefix sum over groups of 16 lanes (4 shuffle steps): exact for
 // lanes 0-15, which are the only ones the pop reads.  A round takes at most
 // 16 ranges (sibling sets of up to 8 nodes fill the warp with 4): measured

@@ -1,4 +1,5 @@
-// walk.cuh -- device helpers shared by the tree walks (project.cu, packet.cu).
+// walk.cuh -- device helpers shared by the tree walks (project.cu, packet.cu,
+// gather.cu).
 #pragma once
 
 #include "mlods_internal.cuh"
@@ -95,5 +96,17 @@ __device__ __forceinline__ Two operator-(Two a, Two b) { return Two{a.x - b.x, a
 __device__ __forceinline__ Two operator*(Two a, Two b) { return Two{a.x * b.x, a.y * b.y}; }
 __device__ __forceinline__ Two operator*(float a, Two b) { return Two{a * b.x, a * b.y}; }
 __device__ __forceinline__ Two fma2(Two a, Two b, Two c) { return Two{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+
+// v + the value o lanes below, where there is one
+__device__ __forceinline__ int add_from_below(int v, int o)
+{
+    int r;
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .s32 t;\n shfl.sync.up.b32 t|p, %1, %2, 0, 0xffffffff;\n"
+        " @p add.s32 t, t, %1;\n @!p mov.s32 t, %1;\n mov.s32 %0, t;\n}"
+        : "=r"(r)
+        : "r"(v), "r"(o));
+    return r;
+}
 
 }  // namespace mlods
