@@ -13,6 +13,7 @@
 // (an upper bound for the k-th distance) and walks the octree with the
 // bounding sphere of each node box, widened by the float rounding of the
 // local frame.  The fit is the reference's CPU one (|u4| < 1e-12).
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -895,23 +896,37 @@ __global__ void global_split_step_kernel(GlobalArgs a, GlobalSplit g, bool last)
     }
 }
 
+// Whole tiles in a range of the points for nq queries: as many ranges as give
+// about eight waves of the resident blocks (the last wave is never full, and the
+// kernel is bound by the exp2 unit as long as blocks are left), at most 64 and
+// their sums within 1 GiB.  Four waves before, of ranges that ended inside a tile
+// and held at least 8: 40k queries on 40k points 9.27 -> 8.92 ms, 17k on 30k 3.34
+// -> 3.05 (5 iterations), 5k on 10k 1.28 -> 0.50, 1 on 5k 1.26 -> 0.19.
+inline int64_t global_range_tiles(int64_t nq, int64_t n_pts, int64_t resident)
+{
+    const int64_t per_block = int64_t(kGlobalThreads) * kGlobalQpt;
+    const int64_t qblocks = (nq + per_block - 1) / per_block;
+    const int64_t tiles = (n_pts + kGlobalTile - 1) / kGlobalTile;
+    if (tiles <= 2) return tiles;  // two launches an iteration cost more than a tile (25 us against 27)
+    int64_t ranges = (8 * resident + qblocks - 1) / qblocks;
+    ranges = std::min(std::min<int64_t>(ranges, 64), std::max<int64_t>((int64_t(1) << 30) / (nq * 72), 1));
+    return (tiles + ranges - 1) / ranges;
+}
+
 // Launches the global projection of one kernel specialisation: the fused
-// kernel when the query tiles fill the GPU about four times over, else the
-// split form over as many point ranges as bring it there.
+// kernel over whole clouds, else the split form.
 template <int KTYPE, int NSIG>
 cudaError_t launch_global_typed(const GlobalArgs& a, int sm_count, cudaStream_t s)
 {
     const int64_t per_block = int64_t(kGlobalThreads) * kGlobalQpt;
     const int64_t qblocks = (a.nq + per_block - 1) / per_block;
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, global_apss_kernel<KTYPE, NSIG>,
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, global_split_sums_kernel<KTYPE, NSIG>,
                                                                   kGlobalThreads, 0);
     if (e != cudaSuccess) return e;
-    const int64_t target = 4 * int64_t(per_sm < 1 ? 1 : per_sm) * sm_count;
-    int64_t chunks = (target + qblocks - 1) / qblocks;
-    const int64_t max_chunks = a.n_pts / (8 * kGlobalTile);  // ranges of at least 2048 points
-    if (chunks > max_chunks) chunks = max_chunks;
-    if (chunks > 64) chunks = 64;
+    const int64_t tiles = (a.n_pts + kGlobalTile - 1) / kGlobalTile;
+    const int64_t range_tiles = global_range_tiles(a.nq, a.n_pts, int64_t(per_sm < 1 ? 1 : per_sm) * sm_count);
+    const int64_t chunks = (tiles + range_tiles - 1) / range_tiles;
     if (chunks <= 1 || a.n_iter < 1) {
         global_apss_kernel<KTYPE, NSIG><<<unsigned(qblocks), kGlobalThreads, 0, s>>>(a);
         note_launch();
@@ -919,7 +934,7 @@ cudaError_t launch_global_typed(const GlobalArgs& a, int sm_count, cudaStream_t 
     }
     GlobalSplit g;
     g.chunks = int(chunks);
-    g.chunk_pts = (a.n_pts + chunks - 1) / chunks;
+    g.chunk_pts = range_tiles * kGlobalTile;
     const size_t part_bytes = size_t(chunks) * size_t(a.nq) * 9 * sizeof(double);
     const size_t state_bytes = size_t(a.nq) * (3 * sizeof(double) + 3 * sizeof(float) + sizeof(uint32_t));
     void* mem = nullptr;
