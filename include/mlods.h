@@ -387,7 +387,8 @@ typedef struct {
     int32_t grid_pct;         /* share of the resident grid launched, 1-100 */
     int32_t line_order;       /* 0: the trees with the most work first; 1: grouped by walk specialisation */
     int64_t solo_min_queries; /* > 0: a tree with at least this many queries runs in a launch of its own
-                                 (the single-tree kernel) before the shared launch of the others; 0: none */
+                                 (the single-tree kernel) before the shared launch of the others; 0: the library's
+                                 choice (two queries per warp: trees that fill the GPU's walks four times over) */
 } mlods_batch_schedule;
 int mlods_batch_create(const mlods_tree* trees, int32_t n_trees, mlods_batch* out);
 int mlods_batch_free(mlods_batch b);

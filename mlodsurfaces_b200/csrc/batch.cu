@@ -199,7 +199,16 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
         b->h_clouds = clouds;
         b->h_offsets.assign(offsets, offsets + n + 1);
     }
-    // the trees with a launch of their own (the largest first) and the rest
+    // the trees with a launch of their own (the largest first) and the rest.
+    // The single-tree kernel reads a tree's arguments at fixed places of the
+    // constant bank, the shared launch by the tree's index, which costs two
+    // queries per warp a tenth (24 clouds of 4k-160k queries: 72.4 ms in one
+    // launch, 69.5 / 66.3 / 65.3 / 65.2 with the trees from 133k / 66k / 33k / 16k
+    // on apart; one query per warp 88.5 or 87.9): without a wish the trees that
+    // fill the GPU's walks four times over go apart, where the empty end of a
+    // launch costs less than that.
+    int64_t solo_min = b->sched.solo_min_queries;
+    if (solo_min <= 0) solo_min = q == 2 ? 4 * project_resident_queries(2, sm_count_for_current_device()) : INT64_MAX;
     std::vector<int> packet, solo;
     std::vector<CloudArgs> qclouds;
     std::vector<int64_t> qbase, qlen;
@@ -208,7 +217,7 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
         if (len == 0) continue;
         if (walks_in_packets(clouds[size_t(i)], q, len, b->sched.reorder != 0)) {
             packet.push_back(i);
-        } else if (b->sched.solo_min_queries > 0 && len >= b->sched.solo_min_queries) {
+        } else if (len >= solo_min) {
             solo.push_back(i);
         } else {
             qclouds.push_back(clouds[size_t(i)]);
