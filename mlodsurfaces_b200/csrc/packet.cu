@@ -39,13 +39,15 @@ constexpr uint32_t kFull = 0xffffffffu;
 constexpr int kPkLevelShift = 24;
 constexpr uint32_t kPkLevelMask = 0xFu;
 // A lane adds about 1200 terms an iteration.  It keeps them in blocks, ended by
-// the ranges up to kPkBlockLevel that its query needs (some 80), and blocks of
-// blocks, ended by those up to kPkSumLevel, so that its sums round about as the
-// other walks' 32 lane sums do: unit normals off FP64 by 1.8e-7 / 1.2e-7 (200k
-// four-Gaussian / 300k torus queries; two per warp 1.7e-7 / 1.0e-7), in one sum
-// 3.8e-7 / 2.7e-7, at 8 % of the time.
-constexpr uint32_t kPkBlockLevel = 5;
-constexpr uint32_t kPkSumLevel = 2;
+// the ranges up to this level that its query needs, and the next block starts
+// from what rounding left out of the total (the fast two-sum's error term), so
+// that only the roundings within a block stay.  Normals off FP64 (rms, 1e-7) for
+// one sum / two plain levels of blocks / this one at 5, 6, 7, 8, every level,
+// beside one query per warp: 400k four-Gaussian queries - / 3.04 / 2.11, 1.71,
+// 1.95, 1.60, 1.60 beside 1.63; 500k rational - / 2.81 / 2.75, 2.64, 2.60, 2.58,
+// 2.58 beside 2.59; 200k four-Gaussian 3.8 in one sum beside 1.7.  2M queries:
+// 132 / 143.5 / 140.2, 140.9, 141.6, 142.7, 144.8 ms.
+constexpr uint32_t kPkBlockLevel = 8;
 constexpr uint32_t kPkNoBlend = 1u << 31;
 constexpr uint32_t kPkLastOnly = 1u << 30;  // CPU rule multi-point leaf: only the last point is weighted
 // A range holds at most 8 nodes (a multi-point leaf's points push nothing) and
@@ -84,7 +86,6 @@ struct __align__(16) PacketWarp {
     float4 par[4];   // those of the node above
     uint4 ent[kPkCap];
     float f[kPkRows][32];
-    float block[9][32];
 };
 
 struct Moments {
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kPkThreads, kPkMinBlocks) mlod_packet_kernel(P
             Moments acc;
             float sum[9];
 #pragma unroll
-            for (int k = 0; k < 9; ++k) acc.v[k] = sum[k] = sm.block[k][lane] = 0.f;
+            for (int k = 0; k < 9; ++k) acc.v[k] = sum[k] = 0.f;
             uint32_t n_visits = 0, n_evals = 0, n_rounds = 0;
             int top = 1;
             if (lane == 0) sm.ent[0] = make_uint4(0u, 1u | kPkNoBlend, live_all, 0u);  // the root alone
@@ -176,13 +177,9 @@ __global__ void __launch_bounds__(kPkThreads, kPkMinBlocks) mlod_packet_kernel(P
                 if (level <= kPkBlockLevel && live) {
 #pragma unroll
                     for (int k = 0; k < 9; ++k) {
-                        float b = sm.block[k][lane] + acc.v[k];
-                        acc.v[k] = 0.f;
-                        if (level <= kPkSumLevel) {
-                            sum[k] += b;
-                            b = 0.f;
-                        }
-                        sm.block[k][lane] = b;
+                        const float t = sum[k] + acc.v[k];
+                        acc.v[k] -= t - sum[k];  // what the sum's rounding left out
+                        sum[k] = t;
                     }
                 }
                 n_visits += uint32_t(__popc(e.z) * left);
@@ -272,7 +269,7 @@ __global__ void __launch_bounds__(kPkThreads, kPkMinBlocks) mlod_packet_kernel(P
             rounds += n_rounds;
             iterations += __popc(live_all);
 #pragma unroll
-            for (int k = 0; k < 9; ++k) sum[k] += sm.block[k][lane] + acc.v[k];
+            for (int k = 0; k < 9; ++k) sum[k] += acc.v[k];
             if (!done) {
                 double xr[3] = {0.0, 0.0, 0.0};
                 if (!fit_sphere(sum, double(c.step_max), gpu_rule, xr, nrm)) {
