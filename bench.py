@@ -1094,7 +1094,7 @@ def run_batch(args, rank: int = 0, world: int = 1):
     if any_solo:
         one = min((c for c in tune_results if c["solo_min_queries"] == 0), key=lambda c: c["ms"])
         b.set_schedule(one["queries_per_warp"], bool(one["reorder"]), one["grid_pct"],
-                       one["line_order"] == "by specialisation", 0)
+                       one["line_order"] == "by specialisation", 1 << 62)
         b.project_device(counts, d_q, d_p, d_n, iters, use_graph=True)
         one_ms = []
         for _ in range(args.steps):
@@ -1171,9 +1171,9 @@ def run_batch(args, rank: int = 0, world: int = 1):
                    "parallelism": (f"whole clouds per GPU, {world} GPUs (rank 0: {len(clouds)} clouds, "
                                    f"{n_points} points)") if world > 1 else "1 GPU",
                    "kernels": "Gaussian / multi-Gaussian / rational drawn per cloud", "tree_depths": "7..10",
-                   "launch": "the Morton ordering, then one persistent queue-kernel launch for every cloud "
-                             "(or launches of their own for the largest clouds first, when the tuner picks it), "
-                             "captured in one CUDA graph",
+                   "launch": "the Morton ordering, launches of their own for the clouds that fill the GPU's walks "
+                             "(those the schedule names, or at the library's choice), then one persistent "
+                             "queue-kernel launch for the others, captured in one CUDA graph",
                    "l2": "L2 flushed (256 MB write) before every timed step"},
         "schedule": {"queries_per_warp": st["queries_per_warp"],
                      "query_order": "Morton" if st["reorder"] else "input", "grid_pct": st["grid_pct"],

@@ -417,7 +417,7 @@ int mlods_batch_tune_results(mlods_batch b, int32_t max_candidates, mlods_batch_
  * blend rule, query ordering and convergence mode apply), but the call
  * allocates no device memory: its scratch (query order, sort buffers, work
  * counter) lives in one fixed array of about 13 MB that the library's module
- * holds on each device, instead of the tree's lazily grown cudaMalloc buffer.
+ * holds on each device, instead of the tree's lazily grown pool buffer.
  * For callers that must not allocate at call time (fixed memory budget, an
  * allocator that owns the free memory, start-up-only footprint).
  *   - n is at most MLODS_NOALLOC_MAX_QUERIES per call; larger n returns

@@ -1,4 +1,4 @@
-// batch.cu -- many resident trees projected by ONE persistent launch.
+// batch.cu -- many resident trees projected by one set of persistent launches.
 //
 // No counterpart in the reference (one tree, one launch per call).  The batch
 // orders each tree's queries in Morton order (one radix sort over all of

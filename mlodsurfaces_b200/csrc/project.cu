@@ -25,9 +25,11 @@
 // S_pp = sum c (cpp + |pbar - q|^2 m0)), reduced across the warp, and the
 // algebraic sphere is solved in double (Fastapss.cu:354-395).
 //
-// Two kernels share the per-query walk: one for a single tree, and a batched
-// one that serves many resident trees (each with its own kernel and options)
-// from one persistent launch.
+// The walk has a narrow form (32 nodes a round, one, two or four queries per
+// warp) and a wide one (64 nodes a round, one query per warp); packet.cu holds
+// a third with a query per lane.  Two kernels here share the walks: one for a
+// single tree, and a batched one that serves many resident trees (each with its
+// own kernel and options) from one persistent launch.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
