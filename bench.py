@@ -194,28 +194,27 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
-# DRAM bytes (read + write) of one projection launch of the default workload
-# (2M points, 2M queries, 10 iterations), from a single-pass ncu capture of
-# dram__bytes_read.sum + dram__bytes_write.sum of mlod_project_kernel on that
-# workload (python bench.py --steps 2 --warmup 1 under ncu --metrics ...).
-PROFILED_TRAFFIC = {("precision", 2_000_000, 10): 503.71e6 + 146.34e6}
+# DRAM bytes (read + write) of one projection of the default workload (2M
+# points, 2M queries, 10 iterations): the two launches of mlod_packet_kernel
+# (the first iteration, the other nine) in a single-pass ncu capture of
+# dram__bytes_read.sum + dram__bytes_write.sum on that workload (python
+# bench.py --steps 2 --warmup 3 under ncu --metrics ...).
+PROFILED_TRAFFIC = {("precision", 2_000_000, 10): 501.33e6 + 238.35e6 + 637.26e6 + 269.08e6}
 PRUNE_TOLS = (1e-6, 1e-3, 1e-1)  # tolerances of the reported kernel-weight pruning runs
-# Counters of the same kernel from a `--set full` capture of the workload
-# scaled to 200k points (one launch, -k mlod_project -s 3 -c 1): the limits
-# the algorithmic-bytes figure does not show.
+# Counters of the same kernel from an ncu capture of the workload scaled to
+# 800k points and queries (the launch of iterations 2 and 3 of three): the
+# limits the algorithmic-bytes figure does not show.
 PROFILED_COUNTERS = {
-    "precision": {"capture": "ncu --set full, precision workload at 200k points, two queries per warp (packed "
-                             "f32x2 arithmetic), one launch",
-                  "issue_slots_active_pct": 76.7, "warp_instructions_per_query_node_visit": 6.61,
-                  "threads_active_per_instruction": 28.74, "warps_active_per_sm": 27.6,
-                  "l2_sector_throughput_gbs": 4193.0, "l2_throughput_pct": 15.7, "l2_hit_rate_pct": 99.09,
-                  "l1_throughput_pct": 66.8, "fp32_fma_pipe_cycles_pct": 35.9, "alu_pipe_pct": 56.5,
-                  "xu_pipe_pct": 39.9, "fp64_pipe_pct": 3.13,
-                  "top_stalls_per_issue": {"wait": 2.25, "short_scoreboard": 1.67, "not_selected": 1.66,
-                                           "long_scoreboard": 0.75}},
+    "precision": {"capture": "ncu sections, precision workload at 800k points, mlod_packet_kernel, iterations 2-3 of 3",
+                  "issue_slots_active_pct": 80.3, "warp_instructions_per_query_node_visit": 5.9,
+                  "threads_active_per_instruction": 31.59, "warps_active_per_sm": 26.8,
+                  "l2_throughput_pct": 10.7, "l2_hit_rate_pct": 98.25, "l1_throughput_pct": 45.5,
+                  "fp32_fma_pipe_cycles_pct": 40.7, "alu_pipe_pct": 33.6, "xu_pipe_pct": 42.8, "fp64_pipe_pct": 0.19,
+                  "top_stalls_per_issue": {"wait": 2.17, "not_selected": 2.04, "short_scoreboard": 1.28,
+                                           "long_scoreboard": 0.58}},
 }
 # L2 sector throughput peak of the B200 as ncu reports it (lts__t_sectors:
-# 3 sectors per cycle per slice at the L2 clock), from the capture above:
+# 3 sectors per cycle per slice at the L2 clock), from a capture of the walk:
 # 131.05 sectors/ns at 12.09 % of peak
 L2_PEAK_GBS = 131.05 * 32 / 0.1209
 
@@ -552,8 +551,8 @@ def run_ours(args, rank, world, local_rank):
     mean_visits = statistics.mean(visits)
     bytes_per_launch = len(q) * (12 + 24) + 64 * mean_visits
     roof_note = (f"algorithmic bytes = 36 per query + 64 per node visit ({mean_visits / len(q) / args.iters:.0f}"
-                 f" visits per query-iteration, the reference walk's); a warp walking two queries loads a node they "
-                 f"share once, so frac can exceed 1 (node_evaluations: the bytes of the loads made); traffic = DRAM "
+                 f" visits per query-iteration, the reference walk's); queries that share a walk load "
+                 f"its nodes once, so frac can exceed 1 (node_evaluations: the bytes of the loads made); traffic = DRAM "
                  f"bytes per launch from ncu: the node arrays are read from DRAM about once, later visits hit L1/L2")
     if spec.get("knn"):  # the k neighbours' positions and normals, every iteration
         bytes_per_launch = len(q) * (12 + 24) + len(q) * args.iters * spec["knn"] * 24
@@ -606,6 +605,13 @@ def run_ours(args, rank, world, local_rank):
                             f"peak = 148 SMs x 16 exp2 per SM per clock (nominal) at the median sampled SM clock; "
                             f"the points stream from L2 through shared memory (HBM is not the bound)"}
 
+    lane_use = None
+    if not spec.get("knn") and not spec.get("global"):
+        # nodes on the lanes, or (a node evaluated for more queries than the
+        # four such a warp walks at most) queries on them
+        ev = statistics.mean(lane_visits)
+        lane_use = mean_visits / (32.0 * ev) if mean_visits > 4.0 * ev else ev / (32.0 * statistics.mean(rounds))
+
     result = {
         "metric": METRIC,
         "value": value,
@@ -639,7 +645,7 @@ def run_ours(args, rank, world, local_rank):
         "traversal": None if spec.get("knn") or spec.get("global") else {
             "visits_per_query_iteration": mean_visits / len(q) / args.iters,
             "node_evaluations_per_query_iteration": statistics.mean(lane_visits) / len(q) / args.iters,
-            "lane_utilisation": statistics.mean(lane_visits) / (32.0 * statistics.mean(rounds)),
+            "lane_utilisation": lane_use,
             "max_stack_ranges": max_stack,
             "note": "visits: nodes each query's walk touches (the reference's traversal); node evaluations: "
                     "what the warps computed, a node shared by the queries of one warp's walk counted once"},

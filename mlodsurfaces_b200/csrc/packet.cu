@@ -12,10 +12,11 @@
 // f_n w_n sum_c (1 - beta_c) rho_c times its own moments S_n once its children
 // have been evaluated.
 //
-// About 104 instructions a node for 32 queries, of which 0.74 need it, against
-// 342 for 50 query-nodes with two queries per warp and 395 for 48 in the wide
-// walk: 2M four-Gaussian queries, 10 iterations, 144 ms (two per warp 172, one
-// 218); 500k rational, 5 iterations, 8.1 ms (9.6, 14.2).  Two queries or two
+// Of a packet's 32 queries 0.71 need the node they evaluate; 5.9 instructions of
+// a warp for each query that does, all in all (80 % of the issue slots), against
+// 6.8 with two queries per warp and 8.2 in the wide walk: 2M four-Gaussian
+// queries, 10 iterations, 143 ms (two per warp 172, one 218); 500k rational, 5
+// iterations, 8.2 ms (9.6, 14.2).  Two queries or two
 // children a lane in packed f32x2 instructions issue as many (the operands'
 // pairs cost the moves) and ran at 160-210 ms.
 //
@@ -58,9 +59,9 @@ constexpr int kPkCap = 7 * kMaxTreeDepth + 4;
 // the resident warps.
 constexpr int kPkRows = 24;
 constexpr int kPkThreads = 128;
-// 7 blocks of 4 warps (72 registers): the walk is bound by the latency of its
-// dependent chains as much as by issue (70 % of the slots at 5.2 warps a
-// scheduler).  2M four-Gaussian / 500k rational workload at 6 / 7 / 8 blocks: 156 /
+// 7 blocks of 4 warps (72 registers): the walk is bound by issue (80 % of the
+// slots at 6.7 warps a scheduler) and by the latency of its dependent chains (70 %
+// at 5.2).  2M four-Gaussian / 500k rational workload at 6 / 7 / 8 blocks: 156 /
 // 144 / 145 and 9.0 / 8.1 / 8.6 ms.
 constexpr int kPkMinBlocks = 7;
 // State of a query between two launches of one projection, kept in the output
