@@ -308,7 +308,8 @@ int mlods_dc_evaluate_device(mlods_tree t, int64_t n_cells, const int32_t* d_cel
  * same results in the same order), mlods_mesh_get copies it into the
  * caller's buffers (pinned buffers copy fastest), and
  * mlods_mesh_device_arrays gives its device arrays (float3 positions and
- * normals, uint3 triangles), valid until the mesh is changed or freed. */
+ * normals, uint3 triangles), valid until the mesh is changed or freed.  They
+ * belong to the device's memory pool: another device or process takes a copy. */
 typedef struct mlods_mesh_s* mlods_mesh;
 int mlods_dc_extract(int64_t n_cells, const int32_t* cells, const float* corner_f, const float* cell_vertex,
                      mlods_mesh* out);
