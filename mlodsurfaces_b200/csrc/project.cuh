@@ -135,8 +135,9 @@ struct BatchFrame {
 // query per warp: 350k queries on 350k / 700k points 33.4 / 28.4 ms, not 40.0 /
 // 35.7, 500k rational 8.1, not 14.2, but 150k on 150k 18.1, not 15.6, 200k on
 // 600k 24.9, not 23.9.  Two or four queries per warp already share nodes: 800k on
-// 800k 75.7, not 79.4, 1M-point 51.6, not 59.6, 2M 144, not 172, but 400k on
-// 500k 40.9, not 37.5, and 500k on 2M 48, not 45.  Not with one iteration
+// 800k 75.7, not 79.4, 1M-point 51.6, not 59.6, 2M 143, not 172, but 400k on
+// 500k 40.9, not 37.5, and 500k on 2M 48, not 45; at 650k it hangs on the cloud
+// (four Gaussians on a torus 62.8, not 60.4, on blobs 44.9, not 46.0).  Not with one iteration
 // (walks_wide gives the reason), with pruning, or stopping at a tolerance (a
 // query's end does not fit the state kept between the launches); exact
 // convergence returns the bits of a run without it, which is promised with one
