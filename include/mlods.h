@@ -308,8 +308,7 @@ int mlods_dc_evaluate_device(mlods_tree t, int64_t n_cells, const int32_t* d_cel
  * same results in the same order), mlods_mesh_get copies it into the
  * caller's buffers (pinned buffers copy fastest), and
  * mlods_mesh_device_arrays gives its device arrays (float3 positions and
- * normals, uint3 triangles), valid until the mesh is changed or freed.  They
- * belong to the device's memory pool: another device or process takes a copy. */
+ * normals, uint3 triangles), valid until the mesh is changed or freed. */
 typedef struct mlods_mesh_s* mlods_mesh;
 int mlods_dc_extract(int64_t n_cells, const int32_t* cells, const float* corner_f, const float* cell_vertex,
                      mlods_mesh* out);
@@ -418,7 +417,7 @@ int mlods_batch_tune_results(mlods_batch b, int32_t max_candidates, mlods_batch_
  * blend rule, query ordering and convergence mode apply), but the call
  * allocates no device memory: its scratch (query order, sort buffers, work
  * counter) lives in one fixed array of about 13 MB that the library's module
- * holds on each device, instead of the tree's lazily grown pool buffer.
+ * holds on each device, instead of the tree's lazily grown buffer.
  * For callers that must not allocate at call time (fixed memory budget, an
  * allocator that owns the free memory, start-up-only footprint).
  *   - n is at most MLODS_NOALLOC_MAX_QUERIES per call; larger n returns
@@ -565,9 +564,12 @@ int64_t mlods_kernel_launches(void);
 
 /* Per-call scratch (DC corner fields, grid generation, split global APSS)
  * comes from a stream-ordered memory pool owned by the library, one per
- * device, which keeps up to 8 GiB of freed scratch for the next calls.
- * mlods_release_scratch returns the current device's unused pooled memory to
- * the system (extension; synchronises the device first). */
+ * device, which keeps up to 8 GiB of freed scratch for the next calls.  The
+ * memory of freed trees, batches, meshes and query buffers (cudaMalloc's) is
+ * kept for the next ones, up to 1 GiB a device.  mlods_release_scratch returns
+ * the current device's unused memory of both kinds to the system (extension;
+ * synchronises the device first); an allocation of the library's own that
+ * finds no memory does the same before it fails. */
 int mlods_release_scratch(void);
 
 #ifdef __cplusplus

@@ -7,6 +7,8 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <unordered_map>
+#include <vector>
 
 #include "dc.h"
 #include "gather.cuh"
@@ -39,7 +41,6 @@ int sm_count_for_current_device()
 namespace
 {
 cudaMemPool_t g_pools[64] = {};
-cudaStream_t g_pool_streams[64] = {};  // where durable memory is allocated and freed
 std::mutex g_pools_mu;
 }  // namespace
 
@@ -85,64 +86,226 @@ cudaError_t scratch_free(void* p, cudaStream_t s) { return p ? cudaFreeAsync(p, 
 
 namespace
 {
-// A stream of the library's own on the current device that carries nothing but
-// durable allocations and frees.
-cudaError_t pool_stream(cudaStream_t* out)
+// Blocks freed by the library's objects wait here for the next one of about
+// their size, the oldest giving way beyond this many bytes a device.
+constexpr size_t kDurableKeepBytes = size_t(1) << 30;
+
+struct DurableBlock {
+    void* p;
+    size_t size;
+    void* fence;  // freed first: see durable_free
+    int device;
+};
+struct DurableState {
+    std::mutex mu;
+    std::unordered_map<void*, DurableBlock> live;
+    std::vector<DurableBlock> idle;   // every use has ended; oldest first
+    std::vector<DurableBlock> stuck;  // freed, but the wait was refused
+    void* anchor[64] = {};            // keeps the driver's chunk for small blocks mapped
+};
+// (never destroyed: objects may be freed while the process exits)
+DurableState& durable_state()
 {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lock(g_pools_mu);
-    if (!g_pool_streams[dev]) e = cudaStreamCreateWithFlags(&g_pool_streams[dev], cudaStreamNonBlocking);
-    *out = g_pool_streams[dev];
+    static DurableState& st = *new DurableState();
+    return st;
+}
+
+// Sizes in sixteenths of a power of two, so that clouds and meshes of about the
+// same size use each other's blocks.
+size_t durable_size(size_t bytes)
+{
+    size_t step = 512;
+    while (step * 32 <= bytes) step *= 2;
+    return (bytes + step - 1) / step * step;
+}
+
+// Takes the idle blocks of `dev` beyond `keep` bytes (the oldest) out of the list.
+std::vector<void*> take_idle(DurableState& st, int dev, size_t keep)
+{
+    size_t total = 0;
+    for (const DurableBlock& b : st.idle)
+        if (b.device == dev) total += b.size;
+    std::vector<void*> out;
+    for (auto it = st.idle.begin(); it != st.idle.end() && total > keep;) {
+        if (it->device != dev) {
+            ++it;
+            continue;
+        }
+        total -= it->size;
+        out.push_back(it->p);
+        it = st.idle.erase(it);
+    }
+    return out;
+}
+
+// Waits as cudaFree does for everything on the block's device, then keeps the
+// block for reuse; a refused wait (a stream capture is open) leaves it for a
+// later call.
+cudaError_t settle(DurableBlock b)
+{
+    DurableState& st = durable_state();
+    cudaError_t e = b.fence ? cudaFree(b.fence) : cudaSuccess;
+    std::vector<void*> out;
+    {
+        std::lock_guard<std::mutex> lock(st.mu);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            st.stuck.push_back(b);
+            return e;
+        }
+        b.fence = nullptr;
+        st.idle.push_back(b);
+        out = take_idle(st, b.device, kDurableKeepBytes);
+    }
+    for (void* p : out) {
+        const cudaError_t ef = cudaFree(p);
+        if (e == cudaSuccess) e = ef;
+    }
+    return e;
+}
+
+void settle_stuck(int dev)
+{
+    DurableState& st = durable_state();
+    std::vector<DurableBlock> again;
+    {
+        std::lock_guard<std::mutex> lock(st.mu);
+        for (auto it = st.stuck.begin(); it != st.stuck.end();) {
+            if (it->device == dev) {
+                again.push_back(*it);
+                it = st.stuck.erase(it);
+            } else {
+                ++it;
+            }
+        }
+    }
+    for (const DurableBlock& b : again) settle(b);
+}
+
+// Idle blocks and unused scratch of `dev`, the current device, back to the system.
+cudaError_t give_back(int dev)
+{
+    std::vector<void*> out;
+    {
+        DurableState& st = durable_state();
+        std::lock_guard<std::mutex> lock(st.mu);
+        out = take_idle(st, dev, 0);
+    }
+    cudaError_t e = cudaSuccess;
+    for (void* p : out) {
+        const cudaError_t ef = cudaFree(p);
+        if (e == cudaSuccess) e = ef;
+    }
+    cudaMemPool_t pool = scratch_pool(dev);
+    if (pool) {
+        const cudaError_t ef = cudaMemPoolTrimTo(pool, 0);
+        if (e == cudaSuccess) e = ef;
+    }
     return e;
 }
 }  // namespace
 
-// cudaMalloc costs 0.1-1 ms a call and cudaFree unmaps as slowly, most of the
-// time of a tree's life: build, one projection and free of 1M points 12.9 ->
-// 4.8 ms (4.4 ms of kernels), the depth-7 mesh pipeline 19.3 -> 13.0 ms.  The
-// pool hands the memory out in microseconds (and keeps what is freed, within
-// its release threshold, until mlods_release_scratch).  The waits make the
-// calls behave as cudaMalloc and cudaFree do towards every stream.
+// Memory of the library's objects: cudaMalloc's (so that a mesh's arrays can be
+// mapped by peers and other processes), kept for the next object when one is
+// freed.  cudaMalloc costs 0.1-1 ms a call beyond the smallest sizes and cudaFree
+// unmaps as slowly, most of the time of a tree's life: build, one projection and
+// free of 1M points 12.9 -> 4.8 ms (4.4 ms of kernels), the depth-7 mesh pipeline
+// 19.3 -> 13.0 ms.
+//
+// What cudaMalloc and cudaFree promise holds: a block comes with a small one of
+// its own, its fence.  Allocating the fence is refused where cudaMalloc is (an
+// open stream capture), and freeing it waits for all work on the device, as
+// cudaFree does, before the block can be used again (2 us each).
+// cudaDeviceSynchronize would wait too, but also end another thread's capture,
+// which cudaFree leaves alone unless that capture asks otherwise.
 cudaError_t durable_alloc(void** p, size_t bytes)
 {
     *p = nullptr;
     if (bytes == 0) return cudaSuccess;
-    cudaStream_t s = nullptr;
-    cudaError_t e = pool_stream(&s);
-    if (e == cudaSuccess) e = scratch_alloc(p, bytes, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return e;
+    DurableState& st = durable_state();
+    DurableBlock b = {nullptr, durable_size(bytes), nullptr, 0};
+    cudaError_t e = cudaGetDevice(&b.device);
+    if (e != cudaSuccess) return e;
+    if (b.device < 64) {
+        std::lock_guard<std::mutex> lock(st.mu);
+        if (!st.anchor[b.device]) e = cudaMalloc(&st.anchor[b.device], 256);
+    }
+    if (e == cudaSuccess) e = cudaMalloc(&b.fence, 256);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        give_back(b.device);
+        e = cudaMalloc(&b.fence, 256);
+    }
+    if (e != cudaSuccess) return e;
+    settle_stuck(b.device);
+    {
+        std::lock_guard<std::mutex> lock(st.mu);
+        auto best = st.idle.end();
+        for (auto it = st.idle.begin(); it != st.idle.end(); ++it)
+            if (it->device == b.device && it->size >= bytes && it->size <= b.size + b.size / 4 &&
+                (best == st.idle.end() || it->size < best->size))
+                best = it;
+        if (best != st.idle.end()) {
+            b.p = best->p;
+            b.size = best->size;
+            st.idle.erase(best);
+        }
+    }
+    if (!b.p) {
+        e = cudaMalloc(&b.p, b.size);
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            give_back(b.device);
+            b.size = bytes;
+            e = cudaMalloc(&b.p, b.size);
+        }
+        if (e != cudaSuccess) {
+            cudaFree(b.fence);
+            return e;
+        }
+    }
+    std::lock_guard<std::mutex> lock(st.mu);
+    st.live[b.p] = b;
+    *p = b.p;
+    return cudaSuccess;
 }
 
 cudaError_t durable_free(void* p)
 {
     if (!p) return cudaSuccess;
-    cudaPointerAttributes at;
-    cudaError_t e = cudaPointerGetAttributes(&at, p);
-    if (e != cudaSuccess) return e;
-    DeviceGuard guard(at.device);
-    e = cudaDeviceSynchronize();
-    cudaStream_t s = nullptr;
-    const cudaError_t es = pool_stream(&s);
-    if (es != cudaSuccess) return es;
-    const cudaError_t ef = cudaFreeAsync(p, s);
-    return e != cudaSuccess ? e : ef;
+    DurableState& st = durable_state();
+    DurableBlock b;
+    {
+        std::lock_guard<std::mutex> lock(st.mu);
+        const auto it = st.live.find(p);
+        if (it == st.live.end()) return cudaErrorInvalidValue;
+        b = it->second;
+        st.live.erase(it);
+    }
+    DeviceGuard guard(b.device);
+    if (guard.err != cudaSuccess) return guard.err;
+    const cudaError_t e = settle(b);
+    if (e == cudaSuccess) settle_stuck(b.device);
+    return e;
 }
 
-// Unused memory of the current device's pool back to the system.
+// The current device's unused memory, scratch and the objects', back to the system.
 cudaError_t scratch_release()
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    cudaMemPool_t pool = scratch_pool(dev);
-    if (!pool) return cudaSuccess;
+    bool held = scratch_pool(dev) != nullptr;
+    {
+        DurableState& st = durable_state();
+        std::lock_guard<std::mutex> lock(st.mu);
+        held = held || !st.idle.empty() || !st.stuck.empty();
+    }
+    if (!held) return cudaSuccess;
     e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return e;
-    return cudaMemPoolTrimTo(pool, 0);
+    settle_stuck(dev);
+    return give_back(dev);
 }
 
 namespace

@@ -142,8 +142,8 @@ int sm_count_for_current_device();
 // Stream-ordered scratch memory from the library's pool on the current device.
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 cudaError_t scratch_free(void* p, cudaStream_t s);
-// Memory that outlives the call, from the same pool: ready for every stream on
-// return, freed once everything on its device that may use it has run.
+// Memory that outlives the call, to be used on any stream: durable_free waits for
+// everything on its device as cudaFree does.
 cudaError_t durable_alloc(void** p, size_t bytes);
 cudaError_t durable_free(void* p);
 template <typename T>

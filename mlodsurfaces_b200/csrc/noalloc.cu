@@ -2,8 +2,8 @@
 //
 // mlods_project_device keeps its per-call scratch (the query processing
 // order, the radix-sort buffers that compute it, the work counter and the
-// statistics block) in a buffer owned by the tree, taken from the library's
-// memory pool on the first call and grown whenever a larger batch arrives.  Some callers
+// statistics block) in a buffer owned by the tree, allocated on the first call
+// and grown whenever a larger batch arrives.  Some callers
 // cannot allow that: a frame loop with a fixed device-memory budget, code
 // that runs while a caching allocator owns all free memory, a process that
 // must reach its final footprint at start-up.  mlods_project_device_noalloc
