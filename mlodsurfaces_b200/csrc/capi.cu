@@ -35,49 +35,97 @@ int sm_count_for_current_device()
     return v;
 }
 
+// (the driver's cuCtxGetCurrent + cuCtxGetId, reached through the runtime so that
+// the library does not link the driver library)
+unsigned long long current_context_id()
+{
+    using GetCurrent = int (*)(void**);
+    using GetId = int (*)(void*, unsigned long long*);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<GetCurrent>(f);
+        f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<GetId>(f);
+        (void)cudaGetLastError();
+    });
+    if (!get_current || !get_id) return 0;
+    void* ctx = nullptr;
+    if (get_current(&ctx) != 0 || !ctx) return 0;
+    unsigned long long id = 0;
+    return get_id(ctx, &id) == 0 ? id : 0;
+}
+
+// The same where memory is about to be allocated: makes device `dev`'s context if
+// there is none (a thread's first call, or the first after a cudaDeviceReset).
+static unsigned long long context_id(int dev)
+{
+    unsigned long long id = current_context_id();
+    if (id == 0 && cudaSetDevice(dev) == cudaSuccess) id = current_context_id();
+    return id;
+}
+
 // Stream-ordered scratch from a memory pool owned by the library (one per
 // device), which keeps up to 8 GiB of freed scratch for reuse, so per-call
 // buffers of a few GB cost neither a cudaMalloc nor a synchronising cudaFree.
+// A pool ends with its context (cudaDeviceReset): one for each context.
 namespace
 {
-cudaMemPool_t g_pools[64] = {};
+struct ScratchPool {
+    int device;
+    unsigned long long ctx;
+    cudaMemPool_t pool;
+};
+std::vector<ScratchPool> g_pools;
 std::mutex g_pools_mu;
+
+// The pool of device `dev` in context `ctx` under the lock, or nullptr.
+cudaMemPool_t find_pool(int dev, unsigned long long ctx)
+{
+    for (const ScratchPool& p : g_pools)
+        if (p.device == dev && p.ctx == ctx) return p.pool;
+    return nullptr;
+}
 }  // namespace
 
 // The pool of device `dev`, or nullptr if none was made yet.
 cudaMemPool_t scratch_pool(int dev)
 {
-    if (dev < 0 || dev >= 64) return nullptr;
+    const unsigned long long ctx = current_context_id();
     std::lock_guard<std::mutex> lock(g_pools_mu);
-    return g_pools[dev];
+    return find_pool(dev, ctx);
 }
 
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s)
 {
-    cudaMemPool_t* pools = g_pools;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev >= 64) return cudaMallocAsync(p, bytes, s);
+    const unsigned long long ctx = context_id(dev);
     cudaMemPool_t pool;
     {
         std::lock_guard<std::mutex> lock(g_pools_mu);
-        if (!pools[dev]) {
+        pool = find_pool(dev, ctx);
+        if (!pool) {
             cudaMemPoolProps props = {};
             props.allocType = cudaMemAllocationTypePinned;
             props.handleTypes = cudaMemHandleTypeNone;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
-            e = cudaMemPoolCreate(&pools[dev], &props);
-            if (e != cudaSuccess) {
-                pools[dev] = nullptr;
-                return e;
-            }
+            e = cudaMemPoolCreate(&pool, &props);
+            if (e != cudaSuccess) return e;
+            g_pools.push_back(ScratchPool{dev, ctx, pool});
             uint64_t keep = uint64_t(8) << 30;
-            e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
             if (e != cudaSuccess) return e;
         }
-        pool = pools[dev];
     }
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
@@ -93,15 +141,16 @@ constexpr size_t kDurableKeepBytes = size_t(1) << 30;
 struct DurableBlock {
     void* p;
     size_t size;
-    void* fence;  // freed first: see durable_free
+    void* fence;  // freed first: see durable_alloc
     int device;
+    unsigned long long ctx;  // a block ends with its context
 };
 struct DurableState {
     std::mutex mu;
     std::unordered_map<void*, DurableBlock> live;
     std::vector<DurableBlock> idle;   // every use has ended; oldest first
     std::vector<DurableBlock> stuck;  // freed, but the wait was refused
-    void* anchor[64] = {};            // keeps the driver's chunk for small blocks mapped
+    std::vector<DurableBlock> anchor;  // keeps the driver's chunk for small blocks mapped
 };
 // (never destroyed: objects may be freed while the process exits)
 DurableState& durable_state()
@@ -120,14 +169,14 @@ size_t durable_size(size_t bytes)
 }
 
 // Takes the idle blocks of `dev` beyond `keep` bytes (the oldest) out of the list.
-std::vector<void*> take_idle(DurableState& st, int dev, size_t keep)
+std::vector<void*> take_idle(DurableState& st, int dev, unsigned long long ctx, size_t keep)
 {
     size_t total = 0;
     for (const DurableBlock& b : st.idle)
-        if (b.device == dev) total += b.size;
+        if (b.device == dev && b.ctx == ctx) total += b.size;
     std::vector<void*> out;
     for (auto it = st.idle.begin(); it != st.idle.end() && total > keep;) {
-        if (it->device != dev) {
+        if (it->device != dev || it->ctx != ctx) {
             ++it;
             continue;
         }
@@ -155,7 +204,7 @@ cudaError_t settle(DurableBlock b)
         }
         b.fence = nullptr;
         st.idle.push_back(b);
-        out = take_idle(st, b.device, kDurableKeepBytes);
+        out = take_idle(st, b.device, b.ctx, kDurableKeepBytes);
     }
     for (void* p : out) {
         const cudaError_t ef = cudaFree(p);
@@ -164,14 +213,14 @@ cudaError_t settle(DurableBlock b)
     return e;
 }
 
-void settle_stuck(int dev)
+void settle_stuck(int dev, unsigned long long ctx)
 {
     DurableState& st = durable_state();
     std::vector<DurableBlock> again;
     {
         std::lock_guard<std::mutex> lock(st.mu);
         for (auto it = st.stuck.begin(); it != st.stuck.end();) {
-            if (it->device == dev) {
+            if (it->device == dev && it->ctx == ctx) {
                 again.push_back(*it);
                 it = st.stuck.erase(it);
             } else {
@@ -183,13 +232,13 @@ void settle_stuck(int dev)
 }
 
 // Idle blocks and unused scratch of `dev`, the current device, back to the system.
-cudaError_t give_back(int dev)
+cudaError_t give_back(int dev, unsigned long long ctx)
 {
     std::vector<void*> out;
     {
         DurableState& st = durable_state();
         std::lock_guard<std::mutex> lock(st.mu);
-        out = take_idle(st, dev, 0);
+        out = take_idle(st, dev, ctx, 0);
     }
     cudaError_t e = cudaSuccess;
     for (void* p : out) {
@@ -223,26 +272,32 @@ cudaError_t durable_alloc(void** p, size_t bytes)
     *p = nullptr;
     if (bytes == 0) return cudaSuccess;
     DurableState& st = durable_state();
-    DurableBlock b = {nullptr, durable_size(bytes), nullptr, 0};
+    DurableBlock b = {nullptr, durable_size(bytes), nullptr, 0, 0};
     cudaError_t e = cudaGetDevice(&b.device);
     if (e != cudaSuccess) return e;
-    if (b.device < 64) {
+    b.ctx = context_id(b.device);
+    const auto of_context = [&](const DurableBlock& o) { return o.device == b.device && o.ctx == b.ctx; };
+    {
         std::lock_guard<std::mutex> lock(st.mu);
-        if (!st.anchor[b.device]) e = cudaMalloc(&st.anchor[b.device], 256);
+        if (std::none_of(st.anchor.begin(), st.anchor.end(), of_context)) {
+            DurableBlock a = {nullptr, 256, nullptr, b.device, b.ctx};
+            e = cudaMalloc(&a.p, a.size);
+            if (e == cudaSuccess) st.anchor.push_back(a);
+        }
     }
     if (e == cudaSuccess) e = cudaMalloc(&b.fence, 256);
     if (e == cudaErrorMemoryAllocation) {
         (void)cudaGetLastError();
-        give_back(b.device);
+        give_back(b.device, b.ctx);
         e = cudaMalloc(&b.fence, 256);
     }
     if (e != cudaSuccess) return e;
-    settle_stuck(b.device);
+    settle_stuck(b.device, b.ctx);
     {
         std::lock_guard<std::mutex> lock(st.mu);
         auto best = st.idle.end();
         for (auto it = st.idle.begin(); it != st.idle.end(); ++it)
-            if (it->device == b.device && it->size >= bytes && it->size <= b.size + b.size / 4 &&
+            if (of_context(*it) && it->size >= bytes && it->size <= b.size + b.size / 4 &&
                 (best == st.idle.end() || it->size < best->size))
                 best = it;
         if (best != st.idle.end()) {
@@ -255,7 +310,7 @@ cudaError_t durable_alloc(void** p, size_t bytes)
         e = cudaMalloc(&b.p, b.size);
         if (e == cudaErrorMemoryAllocation) {
             (void)cudaGetLastError();
-            give_back(b.device);
+            give_back(b.device, b.ctx);
             b.size = bytes;
             e = cudaMalloc(&b.p, b.size);
         }
@@ -284,8 +339,15 @@ cudaError_t durable_free(void* p)
     }
     DeviceGuard guard(b.device);
     if (guard.err != cudaSuccess) return guard.err;
-    const cudaError_t e = settle(b);
-    if (e == cudaSuccess) settle_stuck(b.device);
+    // (the block of an object that outlived its context went with it)
+    cudaPointerAttributes at;
+    cudaError_t e = cudaPointerGetAttributes(&at, b.fence);
+    if (e != cudaSuccess || at.type != cudaMemoryTypeDevice) {
+        (void)cudaGetLastError();
+        return cudaErrorInvalidValue;
+    }
+    e = settle(b);
+    if (e == cudaSuccess) settle_stuck(b.device, b.ctx);
     return e;
 }
 
@@ -295,7 +357,11 @@ cudaError_t scratch_release()
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    bool held = scratch_pool(dev) != nullptr;
+    bool held;
+    {
+        std::lock_guard<std::mutex> lock(g_pools_mu);
+        held = !g_pools.empty();
+    }
     {
         DurableState& st = durable_state();
         std::lock_guard<std::mutex> lock(st.mu);
@@ -304,8 +370,9 @@ cudaError_t scratch_release()
     if (!held) return cudaSuccess;
     e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return e;
-    settle_stuck(dev);
-    return give_back(dev);
+    const unsigned long long ctx = current_context_id();
+    settle_stuck(dev, ctx);
+    return give_back(dev, ctx);
 }
 
 namespace

@@ -139,6 +139,9 @@ void note_launch(int n = 1);
 int64_t launches_so_far();
 // Multiprocessor count of the current device (cached per device).
 int sm_count_for_current_device();
+// Identifier of the calling thread's current context, or 0 when there is none or
+// the driver cannot tell.
+unsigned long long current_context_id();
 // Stream-ordered scratch memory from the library's pool on the current device.
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 cudaError_t scratch_free(void* p, cudaStream_t s);

@@ -47,36 +47,6 @@ ScratchSetup g_scratch[kMaxDevices];
 
 inline size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 
-// Identifier of the calling thread's current context (the driver's
-// cuCtxGetCurrent + cuCtxGetId, reached through the runtime so that the
-// library does not link the driver library), or 0 when there is none or the
-// driver cannot tell.
-unsigned long long current_context_id()
-{
-    using GetCurrent = int (*)(void**);
-    using GetId = int (*)(void*, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-        (void)cudaGetLastError();
-    });
-    if (!get_current || !get_id) return 0;
-    void* ctx = nullptr;
-    if (get_current(&ctx) != 0 || !ctx) return 0;
-    unsigned long long id = 0;
-    return get_id(ctx, &id) == 0 ? id : 0;
-}
-
 // Device address of this device's copy of the scratch array.
 int scratch_for_current_device(char** out)
 {

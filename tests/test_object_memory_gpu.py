@@ -1,13 +1,15 @@
 """Memory of trees, batches and meshes: freeing one leaves the stream captures of
-other threads alone, is refused where cudaFree is (and made up for later), and
-mesh arrays can be shared as cudaMalloc's can."""
+other threads alone, is refused where cudaFree is (and made up for later), mesh
+arrays can be shared as cudaMalloc's can, and a device reset ends what is kept."""
 import ctypes as C
+import subprocess
+import sys
 import threading
 
 import numpy as np
 import pytest
 
-from conftest import make_kernel
+from conftest import ROOT, make_kernel
 from mlodsurfaces_b200 import APSSOctree, DCGrid, Fastapss, synth
 from mlodsurfaces_b200 import _capi as capi
 
@@ -118,3 +120,34 @@ def test_mesh_arrays_can_be_shared():
         ok = C.c_int(0)  # CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE
         assert cu.cuPointerGetAttribute(C.byref(ok), 10, C.c_uint64(part.data_ptr())) == 0
         assert ok.value == 1
+
+
+RESET = """
+import ctypes as C
+import numpy as np
+import torch  # noqa: F401 -- brings libcudart
+from mlodsurfaces_b200 import APSSOctree, Fastapss, GlobalAPSS, Kernel, synth
+pts, nrm = synth.torus(20000, seed=1)
+pts = synth.make_tie_free(pts)
+q = synth.perturbed_queries(pts, 0.01, seed=2)[:2000]
+k = Kernel()
+k.type, k.sigma = Kernel.GAUSSIAN, 0.05
+
+def run():
+    t = APSSOctree()
+    t.build(pts, nrm)
+    out = (*Fastapss(t, k).projectCPU(q, 3), *GlobalAPSS(t, k).projectCPU(q, 2))
+    t.free()
+    return out
+
+before = run()
+assert C.CDLL("libcudart.so.12").cudaDeviceReset() == 0
+for _ in range(2):
+    assert all(np.array_equal(a, b) for a, b in zip(run(), before))
+"""
+
+
+def test_works_on_after_a_device_reset():
+    """Kept blocks and the scratch pool end with their context."""
+    res = subprocess.run([sys.executable, "-c", RESET], cwd=ROOT, capture_output=True, text=True, timeout=240)
+    assert res.returncode == 0, res.stderr
