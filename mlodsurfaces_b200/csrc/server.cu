@@ -47,6 +47,7 @@ struct Request {
     int iters = 0;
     bool own_kernel = false;
     mlods::KernelConsts kc{};
+    bool packets = false;  // walks in packets, as mlods_project_host would
     Clock::time_point t_submit, t_done;
     int status = -1;  // -1 pending, else an MLODS_* code
     char error[256] = "";
@@ -242,8 +243,7 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
         int n_solo = 0;
         for (size_t i = 0; i < nc && e == cudaSuccess; ++i) {
             const int64_t len = w.h_offsets[i + 1] - w.h_offsets[i];
-            // the pieces of a request walk as the whole request would
-            const bool packets = walks_in_packets(w.h_clouds[i], qpw, batch[i].r->n, true);
+            const bool packets = batch[i].r->packets;
             if (packets || len >= solo_min) {
                 // a large piece: launches of its own on its slice of the order
                 ProjectArgs pa;
@@ -570,6 +570,15 @@ int mlods_server_submit(mlods_server s, int32_t tree, int64_t n, const float* q,
             delete r;
             return krc;
         }
+    }
+    {
+        // the pieces of a request walk as the whole request would, by its tree's
+        // settings: not by those of the trees that share a batch with it
+        const mlods_tree_s* T = s->trees[size_t(tree)];
+        CloudArgs c;
+        fill_cloud_args(T, c, nullptr, nullptr, nullptr, n_iterations, -1.f, T->params.blend_rule);
+        c.prune_thr = 0.f;
+        r->packets = walks_in_packets(c, std::min(c.qpw, 2), n, T->params.reorder != 0);
     }
     const int64_t bytes = request_bytes(n);
     std::lock_guard<std::mutex> lock(s->mu);
