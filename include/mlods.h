@@ -445,8 +445,11 @@ int mlods_project_device_noalloc(mlods_tree t, int64_t n, const float* d_q, floa
  * project it with one launch of the queue kernel (every request or piece
  * walked with its own tree, kernel and iteration count); results are written
  * to out_pts / out_nrm (either may be NULL), identical to mlods_project_host
- * on the same tree and kernel (with two queries per warp a request cut into
- * pieces pairs its queries within each piece: equal to float rounding).  The
+ * on the same tree and kernel.  Equal to float rounding instead: with two
+ * queries per warp a request cut into pieces, which pairs its queries within
+ * each piece; with one, a request large enough for mlods_project_host to walk
+ * it in packets (mlods_params) cut into pieces of less than 80,000 queries or
+ * two fifths of the tree's points, which are too small for that.  The
  * query and output arrays must stay valid until the ticket is waited for.
  * Memory admission, by device footprint: a batch in flight holds, in the
  * library's stream-ordered pool, 36 bytes of query / result buffers and

@@ -143,8 +143,7 @@ struct BatchFrame {
 // convergence returns the bits of a run without it, which is promised with one
 // query per warp, so there it follows; and so does a call without Morton order
 // (ordered: whether the call asks for it), whose results are promised to be the
-// same: the packets order the queries themselves.  n is the number of queries
-// of the call or request: not what a server cuts from it.
+// same: the packets order the queries themselves.
 constexpr int64_t kPacketMinQueries = 350000;
 inline bool walks_in_packets(const CloudArgs& c, int qpw, int64_t n, bool ordered)
 {

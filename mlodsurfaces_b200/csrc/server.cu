@@ -47,7 +47,8 @@ struct Request {
     int iters = 0;
     bool own_kernel = false;
     mlods::KernelConsts kc{};
-    bool packets = false;  // walks in packets, as mlods_project_host would
+    bool packets = false;  // walks in packets
+    int64_t piece = 0;     // queries of a piece where it does: equal ones
     Clock::time_point t_submit, t_done;
     int status = -1;  // -1 pending, else an MLODS_* code
     char error[256] = "";
@@ -139,6 +140,24 @@ BatchLayout batch_layout(int64_t n, int64_t r)
     L.frames = take(size_t(r) * sizeof(BatchFrame));
     L.total = at;
     return L;
+}
+
+// Whether a request of n queries that runs in pieces of `piece` walks in packets.
+// With one query per warp as mlods_project_host would, so that results are the
+// same bits, unless the pieces are too small: a piece is every other or every
+// tenth query of the request, not a part of the surface, so the queries of its
+// packets lie further apart, and its last packets run alone.  5 iterations, in
+// packets / in the wide walk, ms: 400k queries on 400k points in pieces of 200k
+// 28.6 / 25.9, 134k 28.4 / 24.2, 100k 33 / 25, 66k 53 / 25, 16k 159 / 26; on 40k
+// points of 80k 21.0 / 20.1, 66k 26.3 / 19.1; 600k on 300k points of 120k 38.4 / 34.6,
+// 100k 41.5 / 34.5; 350k on 700k points of 175k 31 / 23; 2M on 1M points of 200k
+// 144 / 132.  The line allows the same bits a tenth.  Queries that share a walk in
+// twos pair within their piece anyway, so there the piece alone decides (1M
+// queries in pieces of 250k 47.8 ms in twos, 56.2 in packets).
+bool serves_in_packets(const CloudArgs& c, int qpw, int64_t n, int64_t piece, bool ordered)
+{
+    if (qpw > 1) return walks_in_packets(c, qpw, piece, ordered);
+    return walks_in_packets(c, qpw, n, ordered) && (piece == n || (piece >= 80000 && 5 * piece >= 2 * c.n_pts));
 }
 
 int64_t batch_bytes(int64_t n, int64_t r) { return n > 0 ? int64_t(batch_layout(n, r).total) : 0; }
@@ -322,7 +341,8 @@ int64_t form_batch(mlods_server_s* S, std::vector<Piece>& batch)
         if (rest <= room) {
             take = rest;
         } else if (batch.empty()) {
-            take = room;  // a piece as large as the batch can hold
+            // a piece as large as the batch can hold, or one of equal pieces
+            take = r->packets ? std::min(room, r->piece) : room;
         } else {
             ++it;         // fits a later batch only: pass over it
             continue;
@@ -572,13 +592,17 @@ int mlods_server_submit(mlods_server s, int32_t tree, int64_t n, const float* q,
         }
     }
     {
-        // the pieces of a request walk as the whole request would, by its tree's
-        // settings: not by those of the trees that share a batch with it
+        // the pieces of a request walk alike, by its tree's settings: not by those
+        // of the trees that share a batch with it
         const mlods_tree_s* T = s->trees[size_t(tree)];
         CloudArgs c;
         fill_cloud_args(T, c, nullptr, nullptr, nullptr, n_iterations, -1.f, T->params.blend_rule);
         c.prune_thr = 0.f;
-        r->packets = walks_in_packets(c, std::min(c.qpw, 2), n, T->params.reorder != 0);
+        const int64_t cap = std::max<int64_t>(
+            std::min(s->cfg.max_batch_queries, queries_within(s->cfg.max_device_bytes, 1)), 1);
+        const int64_t pieces = (n + cap - 1) / cap;
+        r->piece = (n + pieces - 1) / pieces;
+        r->packets = serves_in_packets(c, std::min(c.qpw, 2), n, r->piece, T->params.reorder != 0);
     }
     const int64_t bytes = request_bytes(n);
     std::lock_guard<std::mutex> lock(s->mu);

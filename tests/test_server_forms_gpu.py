@@ -49,3 +49,21 @@ def test_pieces_do_not_follow_their_batch(projectors):
         assert srv.stats()["batches"] < 10  # they did share one
     finally:
         srv.close()
+
+
+def test_small_pieces_do_not_walk_in_packets(projectors):
+    """Pieces that leave most of the GPU idle in packets take the walk of a call
+    of their own size; all pieces of a request take the same."""
+    (f, q), _ = projectors
+    q = q[:400_000]
+    want = alone(f, q, 2)  # in packets
+    small = [alone(f, q[i:i + 5000], 2) for i in range(0, len(q), 5000)]
+    small = [np.concatenate([s[j] for s in small]) for j in (0, 1)]
+    assert not np.array_equal(small[0], want[0])
+    for batch, same in ((1 << 14, small), (79_999, small), (80_000, want), (1 << 18, want)):
+        srv = ProjectionServer([f], n_streams=2, max_batch_queries=batch)
+        try:
+            got = srv.wait(srv.submit(0, q, 2))
+            assert np.array_equal(got[0], same[0]) and np.array_equal(got[1], same[1]), batch
+        finally:
+            srv.close()
