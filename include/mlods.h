@@ -105,8 +105,11 @@ typedef struct mlods_params {
                                  rounding.  mlods_tune_schedule picks it by timing.  Calls of many
                                  queries (about 350,000 on with 1, 800,000 with 2 or 4, two or more
                                  iterations, about as many queries as points) walk in packets of
-                                 32 queries whatever the setting; with 1 a query's result does
-                                 not depend on the others there either. */
+                                 32 queries whatever the setting, and with 1 smaller calls take 32
+                                 or 64 nodes at a time by the settings, the tree's leaves and,
+                                 below a cutoff of 2.5 or with wide leaves, the number of queries.
+                                 With 1 a query's result does not depend on the other queries,
+                                 only its last bits on their number. */
 } mlods_params;
 
 typedef struct mlods_tree_s* mlods_tree;

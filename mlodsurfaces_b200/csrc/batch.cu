@@ -169,8 +169,8 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
             return MLODS_ERR_INVALID;
         }
         // each cloud's arguments address its own slice of the buffers
-        fill_cloud_args(T, clouds[size_t(i)], d_q + 3 * offsets[i], d_p + 3 * offsets[i], d_n + 3 * offsets[i], iters,
-                        -1.f, T->params.blend_rule);
+        fill_cloud_args(T, clouds[size_t(i)], offsets[i + 1] - offsets[i], d_q + 3 * offsets[i], d_p + 3 * offsets[i],
+                        d_n + 3 * offsets[i], iters, -1.f, T->params.blend_rule);
         CloudArgs& c = clouds[size_t(i)];
         c.prune_thr = 0.f;  // the queue kernel walks without pruning
         float ext = 0.f;

@@ -549,7 +549,7 @@ static int ensure_scratch(mlods_tree_s* T, size_t bytes)
     return MLODS_OK;
 }
 
-void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, const float* d_q, float* d_out_p, float* d_out_n,
+void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, int64_t n, const float* d_q, float* d_out_p, float* d_out_n,
                      int iters, float step_max, int rule)
 {
     c.nodes = T->nodes;
@@ -571,6 +571,8 @@ void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, const float* d_q, floa
     c.local_out = (T->params.local_output != 0 && d_out_p != d_q) ? 1 : 0;
     c.qpw = T->params.queries_per_warp;
     c.n_pts = T->n_pts;
+    c.n_nodes = T->n_nodes;
+    c.n_call = n;
     // kernel-weight pruning: a subtree is dropped below prune_tol times the
     // weight of one average sample sitting at the query (w(0) x mean area)
     c.prune_thr = 0.f;
@@ -754,7 +756,7 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
     }
     const int rule = rule_override >= 0 ? rule_override : T->params.blend_rule;
     ProjectArgs a;
-    fill_cloud_args(T, a.cloud, d_q, d_out_p, d_out_n, iters, step_max, rule);
+    fill_cloud_args(T, a.cloud, n, d_q, d_out_p, d_out_n, iters, step_max, rule);
     a.order = d_order;
     a.nq = n;
     a.counter = reinterpret_cast<unsigned int*>(stats + 3);

@@ -135,7 +135,7 @@ extern "C" int mlods_project_device_noalloc(mlods_tree t, int64_t n, const float
     }
     const int rule = t->params.blend_rule;
     ProjectArgs a;
-    fill_cloud_args(t, a.cloud, d_q, d_out_pts, d_out_nrm, n_iterations, step_max, rule);
+    fill_cloud_args(t, a.cloud, n, d_q, d_out_pts, d_out_nrm, n_iterations, step_max, rule);
     a.order = d_order;
     a.nq = n;
     a.counter = reinterpret_cast<unsigned int*>(stats + 3);

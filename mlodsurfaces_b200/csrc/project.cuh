@@ -53,16 +53,41 @@ struct CloudArgs {
     int local_out;          // 1: out_p holds the result relative to (o0, o1, o2)
     int qpw;                // the tree's walk schedule (queries per warp) for launches of its own
     int64_t n_pts;          // points of the tree
+    int64_t n_nodes;        // and its nodes
+    int64_t n_call;         // queries of the whole call or request on this tree
     float prune_thr;        // > 0: kernel-weight pruning threshold (prune_tol * w(0) * mean sample area)
 };
 
-// Whether a one-query-per-warp projection takes the wide walk.  Not with one
+// Whether a projection may take another form than the narrow walk.  Not with one
 // iteration: that is the projection behind the dual-contouring field and the
 // cell grids, whose signs and cells are whole numbers that follow the float
 // sums of the narrow walk bit for bit; and not with pruning, which is a variant
-// of the narrow walk.  The rule looks at nothing that a batch or a server
-// changes, so a query's result does not depend on what it is projected with.
-inline bool walks_wide(const CloudArgs& c) { return c.n_iter >= 2 && !(c.prune_thr > 0.f); }
+// of the narrow walk.
+inline bool walks_freely(const CloudArgs& c) { return c.n_iter >= 2 && !(c.prune_thr > 0.f); }
+
+// Whether a one-query-per-warp projection takes the wide walk.  Where it does not
+// fill its 64 lanes the narrow one is faster (100k queries on 100k points, 3
+// iterations but where said, narrow / wide, ms):
+//  - its stack holds fewer ranges than the narrow walk's for twice the nodes, and
+//    near its end it pops one range a round: cutoff 6 10.3 / 9.7 and 6.6 / 6.1,
+//    9 19.3 / 23.9, 14 39 / 68; min_depth 4 9.6 / 8.3, 5 30.7 / 31.6, 6 110 / 230;
+//  - it takes 32 of the points of a leaf of more a round: 10.2 points a node
+//    11.3 / 10.9, 15.4 11.9 / 13.9, 25 25.0 / 30.7, 87 53 / 78 -- but for calls that it
+//    holds in flight at once (2,368 queries): 25 1k queries 1.29 / 0.79, 3k 1.50 / 1.45,
+//    4k 1.69 / 1.66, 62 1k 2.27 / 1.63, 4k 2.67 / 2.95;
+//  - short walks spend their time in rounds of a few nodes (10 iterations):
+//    cutoff 2.5 6.0 / 6.0 and 8.4 / 7.8, 2 4.6 / 5.0 and 6.1 / 5.9, 1 3.4 / 4.4;
+//    calls of few queries, which are bound by the number of rounds, gain all the
+//    same: cutoff 2 6k queries 0.46 / 0.38, 14k 0.77 / 0.76, 20k 0.98 / 1.01, 50k
+//    2.31 / 2.49; cutoff 1 6k 0.39 / 0.34, 8k 0.44 / 0.44, 14k 0.63 / 0.69.
+// The rule looks at nothing that a batch or a server changes, so a query's result
+// does not depend on what it is projected with, but for the number of queries.
+inline bool walks_wide(const CloudArgs& c)
+{
+    if (!walks_freely(c) || c.cutoff > 6.f || c.min_depth > 4) return false;
+    if (c.n_pts > 10 * c.n_nodes && c.n_call > 2368) return false;
+    return c.cutoff >= 2.5f || c.n_call <= (c.cutoff < 2.f ? 8192 : 16384);
+}
 
 struct ProjectArgs {
     CloudArgs cloud;
@@ -138,7 +163,7 @@ struct BatchFrame {
 // 800k 75.7, not 79.4, 1M-point 51.6, not 59.6, 2M 143, not 172, but 400k on
 // 500k 40.9, not 37.5, and 500k on 2M 48, not 45; at 650k it hangs on the cloud
 // (four Gaussians on a torus 62.8, not 60.4, on blobs 44.9, not 46.0).  Not with one iteration
-// (walks_wide gives the reason), with pruning, or stopping at a tolerance (a
+// (walks_freely gives the reason), with pruning, or stopping at a tolerance (a
 // query's end does not fit the state kept between the launches); exact
 // convergence returns the bits of a run without it, which is promised with one
 // query per warp, so there it follows; and so does a call without Morton order
@@ -147,7 +172,7 @@ struct BatchFrame {
 constexpr int64_t kPacketMinQueries = 350000;
 inline bool walks_in_packets(const CloudArgs& c, int qpw, int64_t n, bool ordered)
 {
-    if (!walks_wide(c) || n >= (int64_t(1) << 32) - 64) return false;
+    if (!walks_freely(c) || n >= (int64_t(1) << 32) - 64) return false;
     if (c.conv_mode != MLODS_CONVERGE_OFF && !(c.conv_mode == MLODS_CONVERGE_EXACT && qpw == 1)) return false;
     return qpw == 1 ? n >= kPacketMinQueries && 2 * n >= c.n_pts : ordered && n >= 800000 && 4 * n >= 3 * c.n_pts;
 }

@@ -234,7 +234,7 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
         mlods_tree_s* T = S->trees[size_t(r->tree)];
         std::memcpy(hq + 3 * off, r->q + 3 * batch[i].off, size_t(batch[i].n) * 12);
         CloudArgs& c = w.h_clouds[i];
-        fill_cloud_args(T, c, dq + 3 * off, dp + 3 * off, dn + 3 * off, r->iters, -1.f, T->params.blend_rule);
+        fill_cloud_args(T, c, r->n, dq + 3 * off, dp + 3 * off, dn + 3 * off, r->iters, -1.f, T->params.blend_rule);
         if (r->own_kernel) c.kc = r->kc;
         c.prune_thr = 0.f;  // the queue kernel walks without pruning
         qpw = std::max(qpw, std::min(c.qpw, 2));
@@ -596,7 +596,7 @@ int mlods_server_submit(mlods_server s, int32_t tree, int64_t n, const float* q,
         // of the trees that share a batch with it
         const mlods_tree_s* T = s->trees[size_t(tree)];
         CloudArgs c;
-        fill_cloud_args(T, c, nullptr, nullptr, nullptr, n_iterations, -1.f, T->params.blend_rule);
+        fill_cloud_args(T, c, n, nullptr, nullptr, nullptr, n_iterations, -1.f, T->params.blend_rule);
         c.prune_thr = 0.f;
         const int64_t cap = std::max<int64_t>(
             std::min(s->cfg.max_batch_queries, queries_within(s->cfg.max_device_bytes, 1)), 1);

@@ -102,7 +102,7 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
                     float step_max, cudaStream_t s, int rule_override = -1, const CallScratch* cs = nullptr);
 struct CloudArgs;
 // Fills the per-tree part of a projection launch.
-void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, const float* d_q, float* d_out_p, float* d_out_n,
+void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, int64_t n, const float* d_q, float* d_out_p, float* d_out_n,
                      int iters, float step_max, int rule);
 int export_tree(mlods_tree_s* T, int32_t* depth, int32_t* parent, int32_t* first_child, int32_t* n_children,
                 int32_t* next_brother, int32_t* leaf_off, int32_t* leaf_cnt, int32_t* perm, float* bmin, float* bmax,
