@@ -215,8 +215,10 @@ int mlods_project_device(mlods_tree t, int64_t n, const float* d_q, float* d_out
  * untimed run of each, and keeps the fastest in the tree's options
  * (mlods_params.queries_per_warp), which every later single-tree projection
  * uses.  *chosen receives it; ms (may be NULL) the three device times in
- * milliseconds (-1 for a skipped one).  The results of the schedules agree to
- * float rounding.  Synchronises. */
+ * milliseconds (-1 for a skipped one).  Where a call of these queries would walk
+ * in packets under every schedule, the walks of other calls are timed, which
+ * the setting does decide.  The results of the schedules agree to float
+ * rounding.  Synchronises. */
 int mlods_tune_schedule(mlods_tree t, int64_t n, const float* d_q, int32_t n_iterations, void* stream,
                         int32_t* chosen, float* ms);
 /* The same on n host queries (xyz floats), staged in library scratch memory. */

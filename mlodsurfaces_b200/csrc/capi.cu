@@ -764,7 +764,7 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
     a.queries_per_warp = T->params.queries_per_warp;
     const int sm = sm_count_for_current_device();
     const auto launch = [&] {
-        return walks_in_packets(a.cloud, a.queries_per_warp, n, reorder)
+        return !T->no_packets && walks_in_packets(a.cloud, a.queries_per_warp, n, reorder)
                    ? launch_mlod_packets(a, reinterpret_cast<uint32_t*>(base), base + al256(size_t(n) * 4), ext, sm, s)
                    : launch_mlod_project(a, T->kc.type, rule, sm, s);
     };
@@ -1160,6 +1160,13 @@ int mlods_tune_schedule(mlods_tree t, int64_t n, const float* d_q, int32_t n_ite
     int best = saved;
     float best_ms = INFINITY;
     int rc = MLODS_OK;
+    // Where every schedule's queries walk in packets the setting decides nothing
+    // about this call, but it stays and decides others (one iteration, pruning,
+    // tolerances, fewer queries): there the walks that it does decide are timed.
+    CloudArgs c;
+    fill_cloud_args(t, c, n, nullptr, nullptr, nullptr, n_iterations, -1.f, t->params.blend_rule);
+    t->no_packets = true;
+    for (const int q : cands) t->no_packets = t->no_packets && walks_in_packets(c, q, n, t->params.reorder != 0);
     for (int i = 0; i < 3 && rc == MLODS_OK; ++i) {
         float this_ms = -1.f;
         if (!(cands[i] == 4 && t->params.prune_tol > 0.f)) {
@@ -1179,6 +1186,7 @@ int mlods_tune_schedule(mlods_tree t, int64_t n, const float* d_q, int32_t n_ite
         }
         if (ms) ms[i] = this_ms;
     }
+    t->no_packets = false;
     t->params.queries_per_warp = rc == MLODS_OK ? best : saved;
     const cudaError_t ef = scratch_free(out, s);
     if (rc != MLODS_OK) return rc;

@@ -40,6 +40,7 @@ struct mlods_tree_s {
     mlods::KernelConsts kc{};
     mlods_params params{};
     bool kernel_set = false;
+    bool no_packets = false;               // while the schedules are timed: walk as the setting says
 
     // reusable scratch for projection (grown on demand)
     void* d_scratch = nullptr;

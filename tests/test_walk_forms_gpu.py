@@ -103,3 +103,20 @@ def test_last_point_alone_of_a_tree_of_one_leaf():
     assert f.last_stats()["overflows"] == 0 and np.isfinite(p).all()
     failed = np.linalg.norm(m, axis=1) < 0.5
     assert ((p[failed] == q[failed]).all(1) | (p[failed] == first[failed]).all(1)).all()
+
+
+def test_tuner_times_what_the_schedule_decides():
+    """From 800,000 queries on every schedule walks in packets; the pick must
+    still be that of the walks without them, where sharing pays."""
+    pts, nrm = synth.torus(60000, seed=61)
+    f, _ = projector(synth.make_tie_free(pts), nrm, 12, 3.0)
+    q = np.concatenate([synth.perturbed_queries(pts, 0.01, seed=s) for s in range(14)])
+    d_q = torch.from_numpy(q).cuda()
+    res = f.tune_schedule(d_q, 2)
+    assert res["queries_per_warp"] > 1 and f.queries_per_warp == res["queries_per_warp"]
+    assert res["ms"][1] > 1.15 * min(res["ms"].values())
+    before = project(f, q, 2)  # and calls still walk in packets
+    st = f.last_stats()
+    assert st["lane_visits"] < st["node_visits"] / 8
+    f.queries_per_warp = 1
+    assert all(np.array_equal(a, b) for a, b in zip(project(f, q, 2), before))
