@@ -1092,15 +1092,15 @@ def run_batch(args, rank: int = 0, world: int = 1):
         torch.distributed.barrier()
     clk = clocks.stop()
     st = b.last_stats()
-    # when the tuned schedule gave clouds launches of their own, the best
+    # when the tuner gave the largest clouds launches of their own, the best
     # schedule that gives none to any but the clouds walked in packets as well
     single = None
     # (every rank takes the same collective steps: the decision is the max over ranks)
-    any_solo = max_over_ranks([1.0 if st["walk_launches"] > 1 else 0.0], world, dev)[0] > 0
+    any_solo = max_over_ranks([1.0 if st["solo_min_queries"] > 0 else 0.0], world, dev)[0] > 0
     if any_solo:
         one = min((c for c in tune_results if c["solo_min_queries"] == 0), key=lambda c: c["ms"])
         b.set_schedule(one["queries_per_warp"], bool(one["reorder"]), one["grid_pct"],
-                       one["line_order"] == "by specialisation", 1 << 62)
+                       one["line_order"] == "by specialisation", 0)
         b.project_device(counts, d_q, d_p, d_n, iters, use_graph=True)
         one_ms = []
         for _ in range(args.steps):
@@ -1114,7 +1114,7 @@ def run_batch(args, rank: int = 0, world: int = 1):
             one_ms.append(e0.elapsed_time(e1))
         one_max = max_over_ranks([sum(one_ms)], world, dev)[0] / len(one_ms)
         single = {"ms_per_step": one_max, "value": all_queries / (one_max / 1e3), "unit": "queries/s",
-                  "schedule": dict(one, solo_min_queries=1 << 62, ms=None), "walk_launches_per_step": b.last_stats()["walk_launches"]}
+                  "schedule": dict(one, ms=None), "walk_launches_per_step": b.last_stats()["walk_launches"]}
         b.set_schedule(st["queries_per_warp"], bool(st["reorder"]), st["grid_pct"],
                        st["line_order"] == "by specialisation", st["solo_min_queries"])
         b.project_device(counts, d_q, d_p, d_n, iters, use_graph=True)  # the tuned outputs again
@@ -1178,7 +1178,7 @@ def run_batch(args, rank: int = 0, world: int = 1):
                                    f"{n_points} points)") if world > 1 else "1 GPU",
                    "kernels": "Gaussian / multi-Gaussian / rational drawn per cloud", "tree_depths": "7..10",
                    "launch": "the Morton ordering, launches of their own for the clouds that fill the GPU's walks "
-                             "(those the schedule names, or at the library's choice), then one persistent "
+                             "(those the schedule names), then one persistent "
                              "queue-kernel launch for the others, captured in one CUDA graph",
                    "l2": "L2 flushed (256 MB write) before every timed step"},
         "schedule": {"queries_per_warp": st["queries_per_warp"],

@@ -360,15 +360,17 @@ int mlods_last_walk_counts(mlods_tree t, int64_t* lane_visits, int64_t* pruned);
 /* ---- batched projection over many resident trees (extension) ---------------
  * No counterpart in the reference, which projects one tree per launch
  * (Fastapss::project, Fastapss.cu:439-455).  A batch holds a fixed list of
- * trees; mlods_batch_project projects, in ONE persistent kernel launch on one
- * stream (after the Morton ordering of the queries), the device query buffer
+ * trees; mlods_batch_project projects, in one persistent kernel launch on one
+ * stream (after the Morton ordering of the queries and, for trees with many,
+ * launches of their own: see mlods_batch_schedule), the device query buffer
  * d_q (float xyz, concatenated per tree: tree i owns queries
  * [offsets[i], offsets[i+1]), offsets is a HOST array of n_trees + 1 entries
  * starting at 0) onto their trees, writing d_out_pts/d_out_nrm in the same
  * layout.  The launch's warps take a tree's queries one or two at a time from
  * a device counter, the trees with the most work first (trees with enough
- * queries to walk in packets do so in two launches of their own before it),
- * and walk them with the tree's own specialisation of the walk (kernel family and terms, blend
+ * queries to walk in packets do so in two launches of their own before it, and
+ * with one query per warp those that take 64 nodes at a time go apart from
+ * those that take 32), and walk them with the tree's own specialisation of the walk (kernel family and terms, blend
  * rule, queries per warp), so trees of any size and kernel share the launch.
  * Every tree must be in MLODS_MODE_MLOD with a kernel set; each tree's own
  * cutoff, min_depth, blend rule and convergence mode apply (pruning does not),
@@ -392,8 +394,9 @@ typedef struct {
     int32_t grid_pct;         /* share of the resident grid launched, 1-100 */
     int32_t line_order;       /* 0: the trees with the most work first; 1: grouped by walk specialisation */
     int64_t solo_min_queries; /* > 0: a tree with at least this many queries runs in a launch of its own
-                                 (the single-tree kernel) before the shared launch of the others; 0: the library's
-                                 choice (two queries per warp: trees that fill the GPU's walks four times over) */
+                                 (the single-tree kernel) before the shared launch of the others; 0: none.  Until a
+                                 schedule is set or tuned: with two queries per warp the trees that fill the GPU's
+                                 walks four times over */
 } mlods_batch_schedule;
 int mlods_batch_create(const mlods_tree* trees, int32_t n_trees, mlods_batch* out);
 int mlods_batch_free(mlods_batch b);

@@ -797,8 +797,7 @@ class FastapssBatch:
     def schedule(self) -> dict:
         """The launch shape in use: walk schedule (queries per warp), Morton
         order (reorder), share of the grid, order of the trees in the launch,
-        and the size from which a tree runs in a launch of its own (0: the
-        library's choice)."""
+        and the size from which a tree runs in a launch of its own (0: none)."""
         sc = capi.mlods_batch_schedule()
         capi.check(self._lib.mlods_batch_get_schedule(self._b, C.byref(sc)))
         return self._schedule_dict(sc)

@@ -38,6 +38,7 @@ struct mlods_batch_s {
     std::vector<int64_t> h_offsets;
     // launch shape (the tuner's pick, or set by the caller)
     mlods_batch_schedule sched{0, 1, 100, mlods::kQueueMostWorkFirst, 0};
+    bool own_solo = true;             // no schedule set yet: solo_min_queries is the library's choice
     int run_qpw = 1;                  // the walk schedule the launches use
     std::vector<int> h_packet;        // trees whose queries walk in packets
     std::vector<int> h_solo;          // the others with a launch of their own
@@ -76,6 +77,23 @@ void drop_graph(mlods_batch_s* b)
     b->exec = nullptr;
     b->graph = nullptr;
     b->g_total = -1;
+}
+
+// The walk schedule of the whole batch: the schedule's, else the largest the
+// trees ask for (the queue kernel walks one or two queries per warp).
+int batch_qpw(const mlods_batch_s* b)
+{
+    int q = b->sched.queries_per_warp;
+    if (!q)
+        for (const mlods_tree_s* T : b->trees) q = std::max(q, T->params.queries_per_warp);
+    return q >= 2 ? 2 : 1;
+}
+
+// The number of queries from which a tree runs in a launch of its own (0: none).
+int64_t solo_min_queries(const mlods_batch_s* b, int qpw)
+{
+    if (!b->own_solo) return b->sched.solo_min_queries;
+    return qpw == 2 ? 4 * project_resident_queries(2, sm_count_for_current_device()) : 0;
 }
 
 // Enqueues the whole batch on s (capturable: no host synchronisation).
@@ -178,12 +196,7 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
         frames[size_t(i)] = BatchFrame{T->origin[0], T->origin[1], T->origin[2], ext > 0.f ? 1.f / ext : 1.f,
                                        uint32_t(i)};
     }
-    // one walk schedule for the whole batch: the schedule's, else the largest
-    // the trees ask for (the queue kernel walks one or two queries per warp)
-    int q = b->sched.queries_per_warp;
-    if (!q)
-        for (const CloudArgs& c : clouds) q = std::max(q, c.qpw);
-    q = q >= 2 ? 2 : 1;
+    const int q = batch_qpw(b);
     if (q != b->run_qpw) drop_graph(b);
     b->run_qpw = q;
     for (CloudArgs& c : clouds) c.qpw = q;
@@ -204,11 +217,10 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
     // constant bank, the shared launch by the tree's index, which costs two
     // queries per warp a tenth (24 clouds of 4k-160k queries: 72.4 ms in one
     // launch, 69.5 / 66.3 / 65.3 / 65.2 with the trees from 133k / 66k / 33k / 16k
-    // on apart; one query per warp 88.5 or 87.9): without a wish the trees that
+    // on apart; one query per warp 88.5 or 87.9): without a schedule the trees that
     // fill the GPU's walks four times over go apart, where the empty end of a
     // launch costs less than that.
-    int64_t solo_min = b->sched.solo_min_queries;
-    if (solo_min <= 0) solo_min = q == 2 ? 4 * project_resident_queries(2, sm_count_for_current_device()) : INT64_MAX;
+    const int64_t solo_min = solo_min_queries(b, q) > 0 ? solo_min_queries(b, q) : INT64_MAX;
     std::vector<int> packet, solo;
     std::vector<CloudArgs> qclouds;
     std::vector<int64_t> qbase, qlen;
@@ -237,7 +249,9 @@ int batch_prepare(mlods_batch_s* b, const int64_t* offsets, const float* d_q, fl
     b->h_qclouds = qclouds;
     b->h_qbase = qbase;
     b->h_qlen = qlen;
-    b->walk_launches = 2 * int(packet.size()) + int(solo.size()) + (qclouds.empty() ? 0 : queue_groups(int(qclouds.size())));
+    const int n_wide = q == 2 ? 0 : int(std::count_if(qclouds.begin(), qclouds.end(), walks_wide));
+    b->walk_launches = 2 * int(packet.size()) + int(solo.size()) + queue_groups(n_wide) +
+                       queue_groups(int(qclouds.size()) - n_wide);
     const size_t need = up256(size_t(total) * 4) + query_order_temp_bytes(total);
     if (b->order_bytes < need) {
         drop_graph(b);
@@ -407,6 +421,7 @@ int mlods_batch_tune(mlods_batch b, const int64_t* offsets, const float* d_q, fl
     int rc = MLODS_OK;
     b->tune_cands.clear();
     b->tune_ms.clear();
+    b->own_solo = false;
     for (const mlods_batch_schedule& c : cands) {
         b->sched = c;
         drop_graph(b);
@@ -470,8 +485,10 @@ int mlods_batch_get_schedule(mlods_batch b, mlods_batch_schedule* out)
         set_last_error("batch_get_schedule: bad arguments");
         return MLODS_ERR_INVALID;
     }
+    MLODS_ON_DEVICE(b->device);
     *out = b->sched;
     out->queries_per_warp = b->sched.queries_per_warp ? b->sched.queries_per_warp : b->run_qpw;
+    out->solo_min_queries = solo_min_queries(b, b->ran ? b->run_qpw : batch_qpw(b));
     return MLODS_OK;
 }
 
@@ -490,6 +507,7 @@ int mlods_batch_set_schedule(mlods_batch b, const mlods_batch_schedule* sched)
         return MLODS_ERR_INVALID;
     }
     b->sched = c;
+    b->own_solo = false;
     drop_graph(b);
     return MLODS_OK;
 }
