@@ -93,7 +93,7 @@ int batch_qpw(const mlods_batch_s* b)
 int64_t solo_min_queries(const mlods_batch_s* b, int qpw)
 {
     if (!b->own_solo) return b->sched.solo_min_queries;
-    return qpw == 2 ? 4 * project_resident_queries(2, sm_count_for_current_device()) : 0;
+    return qpw == 2 ? 4 * project_resident_queries(2, false, sm_count_for_current_device()) : 0;
 }
 
 // Enqueues the whole batch on s (capturable: no host synchronisation).
@@ -403,7 +403,7 @@ int mlods_batch_tune(mlods_batch b, const int64_t* offsets, const float* d_q, fl
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // walk schedule, query order, grid size, order of the trees, and launches
     // of their own for the trees that fill the GPU 4 or 16 times over
-    const int64_t fill = project_resident_queries(2, sm_count_for_current_device());
+    const int64_t fill = project_resident_queries(2, false, sm_count_for_current_device());
     const mlods_batch_schedule cands[] = {
         {1, 1, 100, kQueueMostWorkFirst, 0},        {2, 1, 100, kQueueMostWorkFirst, 0},
         {2, 1, 100, kQueueBySpecialisation, 0},     {2, 0, 100, kQueueMostWorkFirst, 0},

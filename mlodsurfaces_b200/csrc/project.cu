@@ -1373,10 +1373,12 @@ cudaError_t launch_mlod_queue(const QueueArgs& a, int queries_per_warp, int sm_c
     return launch_queue_typed<1, false>(a, rest, counters, sm_count, grid_pct, s);
 }
 
-int64_t project_resident_queries(int queries_per_warp, int sm_count)
+int64_t project_resident_queries(int queries_per_warp, bool wide, int sm_count)
 {
-    const int per_sm = queries_per_warp == 4 ? WalkShape<4>::kMinBlocks
-                                             : (queries_per_warp == 2 ? WalkShape<2>::kMinBlocks : kWideMinBlocks);
+    const int per_sm = queries_per_warp == 4   ? WalkShape<4>::kMinBlocks
+                       : queries_per_warp == 2 ? WalkShape<2>::kMinBlocks
+                       : wide                  ? kWideMinBlocks
+                                               : WalkShape<1>::kMinBlocks;
     return int64_t(per_sm) * (kProjectThreads / 32) * queries_per_warp * sm_count;
 }
 

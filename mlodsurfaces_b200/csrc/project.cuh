@@ -141,8 +141,9 @@ inline int queue_groups(int n_clouds) { return (n_clouds + kQueueMaxClouds - 1) 
 cudaError_t launch_mlod_queue(const QueueArgs& a, int queries_per_warp, int sm_count, int grid_pct, cudaStream_t s);
 
 // Queries the single-tree walk holds in flight when every SM runs its
-// blocks (resident warps x queries per warp).
-int64_t project_resident_queries(int queries_per_warp, int sm_count);
+// blocks (resident warps x queries per warp); wide: one query per warp in the
+// wide walk.
+int64_t project_resident_queries(int queries_per_warp, bool wide, int sm_count);
 
 // Per-cloud frame used to key queries: the cloud's rank in the batch order
 // (clouds of a batch keep their own rank: their slots are their query range)

@@ -113,9 +113,12 @@ inline size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 constexpr int kMaxServeGroups = 64;
 constexpr size_t kStatsBytes = 8 * sizeof(int64_t) + (kMaxServeGroups + 1) * sizeof(uint64_t) +
                                size_t(kMaxServeGroups) * kQueueMaxClouds * sizeof(unsigned int);
-// A piece of at least this many times the queries the walk holds in flight
+// A piece of at least this many times the queries its walk holds in flight
 // on the whole GPU runs in a launch of its own (the single-tree kernel, whose
-// arguments sit in the constant bank) before the shared launch of the rest.
+// arguments sit in the constant bank) before the shared launch of the rest: from
+// 94,720 queries on one a warp, 37,888 in the wide walk (16 requests of 60k, 5
+// iterations, 40.7 ms; with the narrow walk's line, in shared launches, 41.8), where
+// one iteration gains nothing (10.4; 10.2).
 constexpr int64_t kSoloFill = 16;
 
 // Device layout of one batch of n queries from r requests or pieces.
@@ -255,7 +258,6 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
         e = compute_batch_order(dq, total, d_offsets, int(nc), d_frames, true, order, mem + L.temp, w.s);
     if (e == cudaSuccess) {
         const int sm = sm_count_for_current_device();
-        const int64_t solo_min = kSoloFill * project_resident_queries(qpw, sm);
         std::vector<CloudArgs> qclouds;
         std::vector<int64_t> qbase, qlen;
         unsigned int* solo_counters = reinterpret_cast<unsigned int*>(w.d_stats + 8 + kMaxServeGroups + 1);
@@ -263,6 +265,7 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
         for (size_t i = 0; i < nc && e == cudaSuccess; ++i) {
             const int64_t len = w.h_offsets[i + 1] - w.h_offsets[i];
             const bool packets = batch[i].r->packets;
+            const int64_t solo_min = kSoloFill * project_resident_queries(qpw, walks_wide(w.h_clouds[i]), sm);
             if (packets || len >= solo_min) {
                 // a large piece: launches of its own on its slice of the order
                 ProjectArgs pa;
