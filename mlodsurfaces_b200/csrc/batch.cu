@@ -120,18 +120,16 @@ int enqueue(mlods_batch_s* b, const float* d_q, int64_t total, bool timed, cudaS
         pa.order = order ? order + b->h_offsets[size_t(i)] : nullptr;
         pa.order_base = order ? uint32_t(b->h_offsets[size_t(i)]) : 0u;
         pa.nq = b->h_offsets[size_t(i) + 1] - b->h_offsets[size_t(i)];
-        pa.counter = solo_counters++;
+        pa.counter = solo_counters;
+        solo_counters += 2;
         pa.stats = b->d_stats;
         pa.queries_per_warp = b->run_qpw;
         return pa;
     };
     for (const int i : b->h_packet) {
-        const mlods_tree_s* T = b->trees[size_t(i)];
-        float ext = 0.f;
-        for (int a = 0; a < 3; ++a) ext = std::max(ext, T->BB[a] - T->bb[a]);
         void* tmp = static_cast<char*>(b->d_order_buf) + up256(size_t(total) * 4);
         MLODS_CUDA(launch_mlod_packets(solo_args(i), static_cast<uint32_t*>(b->d_order_buf) + b->h_offsets[size_t(i)], tmp,
-                                       ext, sm, s));
+                                       query_box(b->trees[size_t(i)]), false, sm, s));
     }
     for (const int i : b->h_solo) {
         const ProjectArgs pa = solo_args(i);
@@ -344,9 +342,9 @@ int mlods_batch_create(const mlods_tree* trees, int32_t n_trees, mlods_batch* ou
         return cuda_fail(guard.err, "batch_create: select device", __FILE__, __LINE__);
     }
     // statistics, a 64-bit slot counter for each launch group of
-    // kQueueMaxClouds trees, a 32-bit work counter for each tree
+    // kQueueMaxClouds trees, a 32-bit work counter and its companion for each tree
     const size_t n_groups = size_t(queue_groups(n_trees)) + 1;
-    b->stats_bytes = (8 * sizeof(int64_t) + n_groups * sizeof(uint64_t) + size_t(n_trees) * sizeof(unsigned int) +
+    b->stats_bytes = (8 * sizeof(int64_t) + n_groups * sizeof(uint64_t) + size_t(n_trees) * 2 * sizeof(unsigned int) +
                       255) / 256 * 256;
     cudaError_t e = durable_alloc(&b->d_offsets, size_t(n_trees + 1) * sizeof(int64_t));
     if (e == cudaSuccess) e = durable_alloc(&b->d_frames, size_t(n_trees) * sizeof(BatchFrame));

@@ -549,6 +549,18 @@ static int ensure_scratch(mlods_tree_s* T, size_t bytes)
     return MLODS_OK;
 }
 
+QueryBox query_box(const mlods_tree_s* T)
+{
+    QueryBox b;
+    b.extent = 0.f;
+    for (int a = 0; a < 3; ++a) b.extent = std::max(b.extent, T->BB[a] - T->bb[a]);
+    for (int a = 0; a < 3; ++a) {
+        b.lo[a] = T->bb[a] - 0.5f * b.extent;
+        b.hi[a] = T->BB[a] + 0.5f * b.extent;
+    }
+    return b;
+}
+
 void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, int64_t n, const float* d_q, float* d_out_p, float* d_out_n,
                      int iters, float step_max, int rule)
 {
@@ -748,11 +760,10 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
     }
     MLODS_CUDA(cudaMemsetAsync(stats, 0, 8 * sizeof(int64_t), s));
     uint32_t* d_order = nullptr;
-    float ext = 0.f;
-    for (int ax = 0; ax < 3; ++ax) ext = std::max(ext, T->BB[ax] - T->bb[ax]);
+    const QueryBox box = query_box(T);
     if (reorder) {
         d_order = reinterpret_cast<uint32_t*>(base);
-        MLODS_CUDA(compute_query_order(d_q, n, T->origin, ext, d_order, base + al256(size_t(n) * 4), s));
+        MLODS_CUDA(compute_query_order(d_q, n, T->origin, box.extent, d_order, base + al256(size_t(n) * 4), s));
     }
     const int rule = rule_override >= 0 ? rule_override : T->params.blend_rule;
     ProjectArgs a;
@@ -765,7 +776,7 @@ int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p
     const int sm = sm_count_for_current_device();
     const auto launch = [&] {
         return !T->no_packets && walks_in_packets(a.cloud, a.queries_per_warp, n, reorder)
-                   ? launch_mlod_packets(a, reinterpret_cast<uint32_t*>(base), base + al256(size_t(n) * 4), ext, sm, s)
+                   ? launch_mlod_packets(a, reinterpret_cast<uint32_t*>(base), base + al256(size_t(n) * 4), box, false, sm, s)
                    : launch_mlod_project(a, T->kc.type, rule, sm, s);
     };
     if (cs) {

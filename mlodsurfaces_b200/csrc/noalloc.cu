@@ -129,9 +129,7 @@ extern "C" int mlods_project_device_noalloc(mlods_tree t, int64_t n, const float
     if (t->params.reorder != 0 && n > 1) {
         d_order = reinterpret_cast<uint32_t*>(base + kStatsBytes);
         char* tmp = base + kStatsBytes + al256(size_t(n) * 4);
-        float ext = 0.f;
-        for (int a = 0; a < 3; ++a) ext = std::max(ext, t->BB[a] - t->bb[a]);
-        MLODS_CUDA(compute_query_order(d_q, n, t->origin, ext, d_order, tmp, s));
+        MLODS_CUDA(compute_query_order(d_q, n, t->origin, query_box(t).extent, d_order, tmp, s));
     }
     const int rule = t->params.blend_rule;
     ProjectArgs a;
@@ -143,10 +141,8 @@ extern "C" int mlods_project_device_noalloc(mlods_tree t, int64_t n, const float
     a.queries_per_warp = t->params.queries_per_warp;
     const int sm = sm_count_for_current_device();
     if (walks_in_packets(a.cloud, a.queries_per_warp, n, t->params.reorder != 0)) {
-        float ext = 0.f;
-        for (int ax = 0; ax < 3; ++ax) ext = std::max(ext, t->BB[ax] - t->bb[ax]);
         MLODS_CUDA(launch_mlod_packets(a, reinterpret_cast<uint32_t*>(base + kStatsBytes),
-                                       base + kStatsBytes + al256(size_t(n) * 4), ext, sm, s));
+                                       base + kStatsBytes + al256(size_t(n) * 4), query_box(t), false, sm, s));
         return MLODS_OK;
     }
     MLODS_CUDA(launch_mlod_project(a, t->kc.type, rule, sm, s));

@@ -80,6 +80,7 @@ struct PacketArgs {
     int n_iter;             // iterations of this launch
     int resume;             // 1: an earlier launch of this projection left the queries' state in the outputs
     int more;               // 1: another launch goes on from the state this one leaves
+    const unsigned int* outside;  // if set: the launch walks only where packets_pay(*outside, nq)
 };
 
 struct __align__(16) PacketWarp {
@@ -106,9 +107,22 @@ struct Moments {
     }
 };
 
+// Queries outside the box.
+__global__ void count_outside_kernel(const float* __restrict__ q, int64_t n, QueryBox box, unsigned int* __restrict__ outside)
+{
+    unsigned int c = 0;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        const float p[3] = {q[3 * i], q[3 * i + 1], q[3 * i + 2]};
+        c += in_box(box, p) ? 0u : 1u;
+    }
+    c = __reduce_add_sync(kFull, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(outside, c);
+}
+
 template <int KTYPE, int NSIG, int RULE>
 __global__ void __launch_bounds__(kPkThreads, kPkMinBlocks) mlod_packet_kernel(PacketArgs a)
 {
+    if (a.outside && !packets_pay(*a.outside, a.nq)) return;
     constexpr bool gpu_rule = RULE == MLODS_BLEND_GPU;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PacketWarp& sm = reinterpret_cast<PacketWarp*>(smem_raw)[threadIdx.x >> 5];
@@ -347,8 +361,8 @@ cudaError_t launch_packet_rule(const PacketArgs& a, int sm_count, cudaStream_t s
 // One iteration, the order of the queries where it has left them -- on the
 // surface, where neighbours stay neighbours -- and the other iterations: of the
 // union's nodes 0.74 instead of 0.52 are then needed by a query.
-cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* order_temp, float extent, int sm_count,
-                                cudaStream_t s)
+cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* order_temp, const QueryBox& box, bool near,
+                                int sm_count, cudaStream_t s)
 {
     auto launch = [&](const PacketArgs& p) {
         return p.cloud.rule == MLODS_BLEND_GPU ? launch_packet_rule<MLODS_BLEND_GPU>(p, sm_count, s)
@@ -364,16 +378,28 @@ cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* ord
     p.n_iter = 1;
     p.resume = 0;
     p.more = 1;
+    p.outside = nullptr;
     cudaError_t e = cudaSuccess;
     if (!p.order) {
         const double origin[3] = {a.cloud.o0, a.cloud.o1, a.cloud.o2};
-        e = compute_query_order(a.cloud.q_in, a.nq, origin, extent, order, order_temp, s);
+        e = compute_query_order(a.cloud.q_in, a.nq, origin, box.extent, order, order_temp, s);
         p.order = order;
         p.order_base = 0;
     }
+    if (e == cudaSuccess && !near) {
+        count_outside_kernel<<<unsigned(sm_count) * 4, 256, 0, s>>>(a.cloud.q_in, a.nq, box, a.counter + 1);
+        note_launch();
+        e = cudaGetLastError();
+        p.outside = a.counter + 1;
+        ProjectArgs w = a;
+        w.order = p.order;
+        w.order_base = p.order_base;
+        w.outside = p.outside;
+        if (e == cudaSuccess) e = launch_mlod_project(w, w.cloud.kc.type, w.cloud.rule, sm_count, s);
+    }
     if (e == cudaSuccess) e = launch(p);
     const double frame[3] = {0.0, 0.0, 0.0};  // the state is in the tree's frame
-    if (e == cudaSuccess) e = compute_query_order(a.cloud.out_p, a.nq, frame, extent, order, order_temp, s);
+    if (e == cudaSuccess) e = compute_query_order(a.cloud.out_p, a.nq, frame, box.extent, order, order_temp, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), s);
     if (e != cudaSuccess) return e;
     p.order = order;

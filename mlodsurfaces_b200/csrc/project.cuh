@@ -98,7 +98,28 @@ struct ProjectArgs {
                             // [5] query-iterations, [6] lane visits (a node shared by a warp's queries once)
     int queries_per_warp = 1;  // 1, or 2: consecutive queries of `order` share one walk
     uint32_t order_base = 0;   // subtracted from every entry of `order` (a tree's slice of a batch order)
+    const unsigned int* outside = nullptr;  // if set: the walk runs only where packets_pay(*outside, nq) does not hold
 };
+
+// The surroundings of a tree's root box, widened by half its largest extent.
+struct QueryBox {
+    float lo[3], hi[3];
+    float extent;  // the root box's largest
+};
+__host__ __device__ inline bool in_box(const QueryBox& b, const float* q)
+{
+    return q[0] >= b.lo[0] && q[0] <= b.hi[0] && q[1] >= b.lo[1] && q[1] <= b.hi[1] && q[2] >= b.lo[2] && q[2] <= b.hi[2];
+}
+// Whether queries of which `outside` lie outside that box walk in packets where
+// walks_in_packets allows it.  Far from the cloud neighbours in Morton order are
+// no neighbours, and a few packets of queries strewn over the cloud run long after
+// the others: 400k queries on 400k points, 3 iterations, with 0 / 12 / 24 / 35 / 44 /
+// 49 / 70 / 96 % outside in packets 11.7 / 12.3 / 11.6 / 11.8 / 11.2 / 11.3 / 11.6 / 9.4 ms,
+// one query per warp 15.5 / 14.2 / 12.3 / 12.1 / 10.4 / 10.3 / 8.7 / 2.8; 350k on 700k
+// points 12.6 / 13.5 / 12.5 / 12.8 / 12.1 / 12.6 / 13.4 / 11.0, not 14.6 / 13.3 / 11.5 / 11.4 / 9.8 /
+// 9.7 / 8.2 / 2.6; 1M on 1M points, two queries per warp, at 0 / 12 / 18 % 28.4 / 28.6 / 29.6,
+// not 30.0 / 29.1 / 28.3.
+__host__ __device__ inline bool packets_pay(unsigned int outside, int64_t nq) { return 8 * int64_t(outside) <= nq; }
 
 // Many trees in ONE persistent launch.  The queries of cloud c occupy the
 // global range [base[c], base[c] + len[c]) of the concatenated buffers, and
@@ -179,9 +200,12 @@ inline bool walks_in_packets(const CloudArgs& c, int qpw, int64_t n, bool ordere
 }
 // The whole projection in packets: a's launch arguments; the order of the
 // queries (made here where a.order is null) is rewritten after the first
-// iteration (order: a.nq entries, may be a.order; order_temp: query_order_temp_bytes(a.nq) bytes; extent: the root box's largest).
-cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* order_temp, float extent, int sm_count,
-                                cudaStream_t s);
+// iteration (order: a.nq entries, may be a.order; order_temp:
+// query_order_temp_bytes(a.nq) bytes).  Where too many queries lie outside `box`
+// the walk of the setting runs instead, which the device decides (a.counter[1]:
+// their number, zero before launch), unless `near` says that they do not.
+cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* order_temp, const QueryBox& box, bool near,
+                                int sm_count, cudaStream_t s);
 
 cudaError_t launch_mlod_project(const ProjectArgs& a, int ktype, int rule, int sm_count, cudaStream_t s);
 

@@ -108,11 +108,11 @@ namespace
 inline size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 // statistics, a 64-bit slot counter for each launch group of
 // kQueueMaxClouds pieces (max_batch_requests is at most kMaxServeGroups
-// groups), then a 32-bit work counter for each piece that runs in a launch
-// of its own
+// groups), then a 32-bit work counter and its companion for each piece that
+// runs in a launch of its own
 constexpr int kMaxServeGroups = 64;
 constexpr size_t kStatsBytes = 8 * sizeof(int64_t) + (kMaxServeGroups + 1) * sizeof(uint64_t) +
-                               size_t(kMaxServeGroups) * kQueueMaxClouds * sizeof(unsigned int);
+                               size_t(kMaxServeGroups) * kQueueMaxClouds * 2 * sizeof(unsigned int);
 // A piece of at least this many times the queries its walk holds in flight
 // on the whole GPU runs in a launch of its own (the single-tree kernel, whose
 // arguments sit in the constant bank) before the shared launch of the rest: from
@@ -273,14 +273,12 @@ int run_batch(mlods_server_s* S, Worker& w, const std::vector<Piece>& batch)
                 pa.order = order + w.h_offsets[i];
                 pa.order_base = uint32_t(w.h_offsets[i]);
                 pa.nq = len;
-                pa.counter = solo_counters + n_solo++;
+                pa.counter = solo_counters + 2 * n_solo++;
                 pa.stats = w.d_stats;
                 pa.queries_per_warp = qpw;
                 if (packets) {
-                    const mlods_tree_s* T = S->trees[size_t(batch[i].r->tree)];
-                    float ext = 0.f;
-                    for (int a = 0; a < 3; ++a) ext = std::max(ext, T->BB[a] - T->bb[a]);
-                    e = launch_mlod_packets(pa, order + w.h_offsets[i], mem + L.temp, ext, sm, w.s);
+                    e = launch_mlod_packets(pa, order + w.h_offsets[i], mem + L.temp,
+                                            query_box(S->trees[size_t(batch[i].r->tree)]), true, sm, w.s);
                 } else {
                     e = launch_mlod_project(pa, pa.cloud.kc.type, pa.cloud.rule, sm, w.s);
                 }
@@ -606,6 +604,12 @@ int mlods_server_submit(mlods_server s, int32_t tree, int64_t n, const float* q,
         const int64_t pieces = (n + cap - 1) / cap;
         r->piece = (n + pieces - 1) / pieces;
         r->packets = serves_in_packets(c, std::min(c.qpw, 2), n, r->piece, T->params.reorder != 0);
+        if (r->packets) {  // by all of its queries, as the device would
+            const QueryBox box = query_box(T);
+            unsigned int outside = 0;
+            for (int64_t i = 0; i < n; ++i) outside += in_box(box, q + 3 * i) ? 0u : 1u;
+            r->packets = packets_pay(outside, n);
+        }
     }
     const int64_t bytes = request_bytes(n);
     std::lock_guard<std::mutex> lock(s->mu);

@@ -102,7 +102,10 @@ size_t project_call_bytes(const mlods_tree_s* T, int64_t n);
 int project_buffers(mlods_tree_s* T, int64_t n, const float* d_q, float* d_out_p, float* d_out_n, int iters,
                     float step_max, cudaStream_t s, int rule_override = -1, const CallScratch* cs = nullptr);
 struct CloudArgs;
-// Fills the per-tree part of a projection launch.
+// The surroundings of the root box, in world coordinates (project.cuh).
+struct QueryBox;
+QueryBox query_box(const mlods_tree_s* T);
+// Fills the per-tree part of a projection of n queries (of the whole call).
 void fill_cloud_args(const mlods_tree_s* T, CloudArgs& c, int64_t n, const float* d_q, float* d_out_p, float* d_out_n,
                      int iters, float step_max, int rule);
 int export_tree(mlods_tree_s* T, int32_t* depth, int32_t* parent, int32_t* first_child, int32_t* n_children,
