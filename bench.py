@@ -547,49 +547,41 @@ def run_ours(args, rank, world, local_rank):
         f.local_output = False
         f._sync_params()
 
-    # ---- roofline of the projection kernel (algorithmic bytes per launch)
+    # ---- roofline of the projection kernel
     mean_visits = statistics.mean(visits)
-    bytes_per_launch = len(q) * (12 + 24) + 64 * mean_visits
-    roof_note = (f"algorithmic bytes = 36 per query + 64 per node visit ({mean_visits / len(q) / args.iters:.0f}"
-                 f" visits per query-iteration, the reference walk's); queries that share a walk load "
-                 f"its nodes once, so frac can exceed 1 (node_evaluations: the bytes of the loads made); traffic = DRAM "
-                 f"bytes per launch from ncu: the node arrays are read from DRAM about once, later visits hit L1/L2")
-    if spec.get("knn"):  # the k neighbours' positions and normals, every iteration
-        bytes_per_launch = len(q) * (12 + 24) + len(q) * args.iters * spec["knn"] * 24
-        roof_note = (f"algorithmic bytes = 36 per query + {spec['knn']} neighbours x 24 bytes per query-iteration "
-                     f"(the octree walk of the gather is not counted)")
     kms = statistics.mean(kern_ms)
-    achieved = bytes_per_launch / (kms / 1e3) / 1e9
     peak, peak_kind = measured_peak_hbm()
     traffic = PROFILED_TRAFFIC.get((args.workload, n_points_for(args), args.iters))
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "note": f"{roof_note}; peak {peak_kind}"}
-    if not spec.get("knn"):
-        # what actually limits the walk: the node records are reread from
-        # L1/L2, not from DRAM, and the instruction issue is the bound
-        roofline["served_from"] = "L1/L2: the algorithmic node bytes are rereads of records already on chip"
-        roofline["l2"] = {"achieved": achieved, "peak": L2_PEAK_GBS, "unit": "GB/s", "frac": achieved / L2_PEAK_GBS,
-                          "note": "the same algorithmic bytes against the L2 sector peak ncu reports"}
-        # a warp walking several queries loads a node once for all of them:
-        # the bytes of the node evaluations it actually makes
-        ev = statistics.mean(lane_visits)
-        loaded = (len(q) * 36 + 64 * ev) / (kms / 1e3) / 1e9
-        roofline["node_evaluations"] = {
-            "achieved": loaded, "peak": peak, "unit": "GB/s", "frac": loaded / peak,
-            "note": f"36 B per query + 64 B per node evaluation ({ev / len(q) / args.iters:.0f} per query-iteration: "
-                    f"a node the queries of one warp share is loaded once), against the HBM peak"}
-        # flops per query-iteration: per node visit 14 (distance, blend) + 18
-        # (moment terms) + the kernel's (10 per Gaussian term, 20 rational),
-        # and about 60 for the sphere solve
+    if spec.get("knn"):  # the k neighbours' positions and normals, every iteration
+        achieved = (len(q) * (12 + 24) + len(q) * args.iters * spec["knn"] * 24) / (kms / 1e3) / 1e9
+        roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                    "traffic": traffic,
+                    "note": f"algorithmic bytes = 36 per query + {spec['knn']} neighbours x 24 bytes per "
+                            f"query-iteration (the octree walk of the gather is not counted); peak {peak_kind}"}
+    else:
+        # the tree stays in L1/L2 and DRAM idles: the walk is bound by
+        # instruction issue, so the flops it cannot do without are set against
+        # the FP32 lanes.  Per node visit 14 (distance, blend) + 18 (moment
+        # terms) + the kernel's (10 per Gaussian term, 20 rational), and about
+        # 60 for the sphere solve
         k_flops = {0: 10, 1: 20}.get(kernel.type, 10 * len(kernel.sigmas))
         flops = mean_visits * (14 + 18 + k_flops) + 60.0 * len(q) * args.iters
         mhz = clk.get("sm_mhz") or 1965.0
         fp32_peak = 148 * 128 * 2 * mhz / 1e6
-        roofline["fp32"] = {"achieved": flops / (kms / 1e3) / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
-                            "frac": flops / (kms / 1e3) / 1e12 / fp32_peak,
-                            "note": "algorithmic flops (per node visit 14 + 18 + 10 per Gaussian term or 20 "
-                                    "rational; 60 per sphere solve) against 148 SMs x 128 FP32 lanes x 2 at the "
-                                    "median sampled SM clock"}
+        achieved = flops / (kms / 1e3) / 1e12
+        roofline = {"bound": "issue", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
+                    "frac": achieved / fp32_peak, "traffic": traffic,
+                    "note": f"algorithmic flops (per node visit 14 + 18 + 10 per Gaussian term or 20 rational, "
+                            f"{mean_visits / len(q) / args.iters:.0f} visits per query-iteration, the reference "
+                            f"walk's; 60 per sphere solve) against 148 SMs x 128 FP32 lanes x 2 at the median "
+                            f"sampled SM clock; traffic = DRAM bytes per projection from ncu"}
+        # a node that the queries of one warp share is loaded once for all of them
+        ev = statistics.mean(lane_visits)
+        loaded = (len(q) * 36 + 64 * ev) / (kms / 1e3) / 1e9
+        roofline["node_loads"] = {
+            "achieved": loaded, "peak": L2_PEAK_GBS, "unit": "GB/s", "frac": loaded / L2_PEAK_GBS,
+            "note": f"36 B per query + 64 B per node evaluation ({ev / len(q) / args.iters:.0f} per query-iteration), "
+                    f"served by L1 and L2, against the L2 sector peak ncu reports"}
         roofline["measured"] = dict(PROFILED_COUNTERS.get(args.workload, {}))
         if traffic:
             roofline["measured"]["dram_gbs"] = traffic / (kms / 1e3) / 1e9
@@ -604,13 +596,6 @@ def run_ours(args, rank, world, local_rank):
                     "note": f"{len(q)} queries x {len(pts)} points x {args.iters} iterations x {nsig} exp2 per launch; "
                             f"peak = 148 SMs x 16 exp2 per SM per clock (nominal) at the median sampled SM clock; "
                             f"the points stream from L2 through shared memory (HBM is not the bound)"}
-
-    lane_use = None
-    if not spec.get("knn") and not spec.get("global"):
-        # nodes on the lanes, or (a node evaluated for more queries than the
-        # four such a warp walks at most) queries on them
-        ev = statistics.mean(lane_visits)
-        lane_use = mean_visits / (32.0 * ev) if mean_visits > 4.0 * ev else ev / (32.0 * statistics.mean(rounds))
 
     result = {
         "metric": METRIC,
@@ -645,7 +630,8 @@ def run_ours(args, rank, world, local_rank):
         "traversal": None if spec.get("knn") or spec.get("global") else {
             "visits_per_query_iteration": mean_visits / len(q) / args.iters,
             "node_evaluations_per_query_iteration": statistics.mean(lane_visits) / len(q) / args.iters,
-            "lane_utilisation": lane_use,
+            "node_evaluations_per_round": statistics.mean(lane_visits) / statistics.mean(rounds),
+            "queries_per_node_evaluation": mean_visits / statistics.mean(lane_visits),
             "max_stack_ranges": max_stack,
             "note": "visits: nodes each query's walk touches (the reference's traversal); node evaluations: "
                     "what the warps computed, a node shared by the queries of one warp's walk counted once"},

@@ -14,11 +14,11 @@
 //
 // Of a packet's 32 queries 0.71 need the node they evaluate; 5.9 instructions of
 // a warp for each query that does, all in all (80 % of the issue slots), against
-// 6.8 with two queries per warp and 8.2 in the wide walk: 2M four-Gaussian
-// queries, 10 iterations, 143 ms (two per warp 172, one 218); 500k rational, 5
-// iterations, 8.2 ms (9.6, 14.2).  Two queries or two
-// children a lane in packed f32x2 instructions issue as many (the operands'
-// pairs cost the moves) and ran at 160-210 ms.
+// 6.8 with two queries per warp and 8.1 in the wide walk: 2M four-Gaussian
+// queries, 10 iterations, 138 ms (two per warp 158, one 212); 500k rational, 5
+// iterations, 8.3 ms (9.4, 12.8).  Two queries or two children a lane in packed
+// f32x2 instructions issue as many (the operands' pairs cost the moves) and ran at
+// 160-210 ms.
 //
 // A query's sums depend on its own walk only: the union's depth-first order
 // restricted to the nodes a query needs is that query's depth-first order, and
@@ -46,8 +46,8 @@ constexpr uint32_t kPkLevelMask = 0xFu;
 // one sum / two plain levels of blocks / this one at 5, 6, 7, 8, every level,
 // beside one query per warp: 400k four-Gaussian queries - / 3.04 / 2.11, 1.71,
 // 1.95, 1.60, 1.60 beside 1.63; 500k rational - / 2.81 / 2.75, 2.64, 2.60, 2.58,
-// 2.58 beside 2.59; 200k four-Gaussian 3.8 in one sum beside 1.7.  2M queries:
-// 132 / 143.5 / 140.2, 140.9, 141.6, 142.7, 144.8 ms.
+// 2.58 beside 2.59; 200k four-Gaussian 3.8 in one sum beside 1.7.  2M queries at
+// 5, 6, 7, 8, every level: 135.8, 136.6, 137.1, 138.2, 140.7 ms.
 constexpr uint32_t kPkBlockLevel = 8;
 constexpr uint32_t kPkNoBlend = 1u << 31;
 constexpr uint32_t kPkLastOnly = 1u << 30;  // CPU rule multi-point leaf: only the last point is weighted
@@ -61,8 +61,8 @@ constexpr int kPkRows = 24;
 constexpr int kPkThreads = 128;
 // 7 blocks of 4 warps (72 registers): the walk is bound by issue (80 % of the
 // slots at 6.7 warps a scheduler) and by the latency of its dependent chains (70 %
-// at 5.2).  2M four-Gaussian / 500k rational workload at 6 / 7 / 8 blocks: 156 /
-// 144 / 145 and 9.0 / 8.1 / 8.6 ms.
+// at 5.2).  2M four-Gaussian / 500k rational workload at 6 / 7 / 8 blocks: 155 /
+// 138 / 141 and 9.2 / 8.3 / 8.8 ms.
 constexpr int kPkMinBlocks = 7;
 // State of a query between two launches of one projection, kept in the output
 // buffers: the iterate in the local frame, or (this pattern in the normal's

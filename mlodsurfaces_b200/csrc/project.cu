@@ -701,12 +701,15 @@ __device__ __forceinline__ void project_packed(const CloudArgs& c, const uint32_
 // The wide walk pops up to 64 nodes a round: two groups of whole sibling ranges
 // of at most 32 nodes, lane l evaluating node l of each.  The pop, the scan and
 // the loop are paid once for twice the nodes and a query's chain of rounds is
-// half as long, which bounds calls of a few thousand queries: 1,000 queries,
-// 10 iterations 381 -> 204 us, 10,000 960 -> 850 us.  Calls that fill the GPU
-// gain less (100k 11.9 -> 9.9 ms, 2M four-Gaussian 245 -> 218 ms): there the
-// node loads keep the L1 data path two thirds busy, 2.1 wavefronts a visit.
-// 4 blocks per SM (128 registers) against 5 / 6 / 7: 218 / 229 / 238 / 255 ms,
-// since every resident warp's stack takes L1 away from the nodes.
+// half as long, which bounds calls of a few thousand queries: 10 iterations of
+// 1,000 queries 370 -> 200 us, of 10,000 880 -> 850 us (1,000: a warp issues every
+// 4.8 cycles, of which it waits 1.6 on its own instructions, 1.0 on shuffles and
+// shared memory, 0.7 on node loads; a round is 364 instructions, 1.2 us).  Calls
+// that fill the GPU gain nothing (100k 9.8 / 9.8 ms, four Gaussians 10.0 / 9.95, 2M
+// 211 / 212): issue is 65 % busy there and the node loads keep the L1 data path at
+// 68 %.  4 blocks per SM (128 registers) against 5 / 6 / 7: 2M 212 / 208 / 245 / 247
+// ms, 1,000 queries 0.20 / 0.21 / 0.26 / 0.26, since every resident warp's stack takes
+// L1 away from the nodes.
 
 template <int CAP>
 struct WideStack {

@@ -178,14 +178,16 @@ struct BatchFrame {
 // Whether a projection of n queries runs in packets of 32 (packet.cu).  Where
 // the packets fill the GPU several times over (148 SMs x 28 warps x 32 queries =
 // 133k; the last packets run alone for about 3 ms) and the queries lie about as
-// close as the points, so that neighbours need the same nodes.  Against one
-// query per warp: 350k queries on 350k / 700k points 33.4 / 28.4 ms, not 40.0 /
-// 35.7, 500k rational 8.1, not 14.2, but 150k on 150k 18.1, not 15.6, 200k on
-// 600k 24.9, not 23.9.  Two or four queries per warp already share nodes: 800k on
-// 800k 75.7, not 79.4, 1M-point 51.6, not 59.6, 2M 143, not 172, but 400k on
-// 500k 40.9, not 37.5, and 500k on 2M 48, not 45; at 650k it hangs on the cloud
-// (four Gaussians on a torus 62.8, not 60.4, on blobs 44.9, not 46.0).  Not with one iteration
-// (walks_freely gives the reason), with pruning, or stopping at a tolerance (a
+// close as the points, so that neighbours need the same nodes.  10 iterations on
+// the torus / blobs (four Gaussians) / knot (rational), packets, not one query per
+// warp: 350k queries on 350k points 34.0 / 25.5 / 14.1 ms, not 40.3 / 30.4 / 18.4, on
+// 700k points 42.1 / 31.8 / 16.9, not 43.7 / 32.8 / 19.6, but 150k on 150k 18.0 / 12.8 /
+// 7.2, not 15.7 / 12.0 / 7.4, 200k on 600k 27.9 / 24.0 / 12.4, not 24.6 / 18.5 / 11.1.
+// Two or four queries per warp already share nodes: 800k on 800k 74.3 / 53.5 / 29.5,
+// not 76.2 / 55.4 / 33.5 with two, 1M on 1M 93.0 / 66.4 / 35.9, not 98.3 / 71.4 / 42.8, but
+// 400k on 500k 41.1 / 30.5 / 16.3, not 36.1 / 26.3 / 16.2, 500k on 2M 71.9 / 51.8 / 29.2,
+// not 56.7 / 41.3 / 24.2; 650k on 650k 60.1 / 45.1 / 24.2, not 60.2 / 43.7 / 26.7.  Not
+// with one iteration (walks_freely gives the reason), with pruning, or stopping at a tolerance (a
 // query's end does not fit the state kept between the launches); exact
 // convergence returns the bits of a run without it, which is promised with one
 // query per warp, so there it follows; and so does a call without Morton order
