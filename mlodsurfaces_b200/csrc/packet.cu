@@ -119,6 +119,14 @@ __global__ void count_outside_kernel(const float* __restrict__ q, int64_t n, Que
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(outside, c);
 }
 
+// The other walk's work counter: at its end, so that its warps find nothing to
+// do, where the packets will walk (a look at `outside` in those kernels cost calls
+// of a thousand queries 1 %).
+__global__ void end_counter_kernel(const unsigned int* __restrict__ outside, int64_t nq, unsigned int* __restrict__ counter)
+{
+    *counter = packets_pay(*outside, nq) ? (unsigned int)nq : 0u;
+}
+
 template <int KTYPE, int NSIG, int RULE>
 __global__ void __launch_bounds__(kPkThreads, kPkMinBlocks) mlod_packet_kernel(PacketArgs a)
 {
@@ -390,12 +398,16 @@ cudaError_t launch_mlod_packets(const ProjectArgs& a, uint32_t* order, void* ord
         count_outside_kernel<<<unsigned(sm_count) * 4, 256, 0, s>>>(a.cloud.q_in, a.nq, box, a.counter + 1);
         note_launch();
         e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
         p.outside = a.counter + 1;
+        end_counter_kernel<<<1, 1, 0, s>>>(p.outside, a.nq, a.counter);
+        note_launch();
+        e = cudaGetLastError();
         ProjectArgs w = a;
         w.order = p.order;
         w.order_base = p.order_base;
-        w.outside = p.outside;
         if (e == cudaSuccess) e = launch_mlod_project(w, w.cloud.kc.type, w.cloud.rule, sm_count, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), s);
     }
     if (e == cudaSuccess) e = launch(p);
     const double frame[3] = {0.0, 0.0, 0.0};  // the state is in the tree's frame

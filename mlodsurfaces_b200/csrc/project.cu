@@ -987,7 +987,6 @@ struct WalkShape {
 template <int KTYPE, int NSIG, int RULE>
 __global__ void __launch_bounds__(kProjectThreads, kWideMinBlocks) mlod_wide_kernel(ProjectArgs a)
 {
-    if (a.outside && packets_pay(*a.outside, a.nq)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     WideStack<kWideCap>& st = reinterpret_cast<WideStack<kWideCap>*>(smem_raw)[threadIdx.x >> 5];
@@ -1007,7 +1006,6 @@ __global__ void __launch_bounds__(kProjectThreads, kWideMinBlocks) mlod_wide_ker
 template <int KTYPE, int NSIG, int RULE, int QPW, bool PRUNE>
 __global__ void __launch_bounds__(kProjectThreads, WalkShape<QPW>::kMinBlocks) mlod_project_kernel(ProjectArgs a)
 {
-    if (a.outside && packets_pay(*a.outside, a.nq)) return;
     constexpr int CAP = WalkShape<QPW>::kCap;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;

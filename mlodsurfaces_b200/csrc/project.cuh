@@ -98,7 +98,6 @@ struct ProjectArgs {
                             // [5] query-iterations, [6] lane visits (a node shared by a warp's queries once)
     int queries_per_warp = 1;  // 1, or 2: consecutive queries of `order` share one walk
     uint32_t order_base = 0;   // subtracted from every entry of `order` (a tree's slice of a batch order)
-    const unsigned int* outside = nullptr;  // if set: the walk runs only where packets_pay(*outside, nq) does not hold
 };
 
 // The surroundings of a tree's root box, widened by half its largest extent.
