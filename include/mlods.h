@@ -108,8 +108,7 @@ typedef struct mlods_params {
                                  them outside the root box widened by half its extent) walk in
                                  packets of 32 queries whatever the setting, and with 1 smaller
                                  calls take 32 or 64 nodes at a time by the settings, the tree's
-                                 leaves and, below a cutoff of 2.5 or with wide leaves, the number
-                                 of queries.  With 1 a query's result does not depend on the other
+                                 leaves and the number of queries.  With 1 a query's result does not depend on the other
                                  queries, only its last bits on how many there are (in large calls
                                  also on how many lie far off). */
 } mlods_params;

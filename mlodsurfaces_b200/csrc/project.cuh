@@ -67,14 +67,15 @@ inline bool walks_freely(const CloudArgs& c) { return c.n_iter >= 2 && !(c.prune
 
 // Whether a one-query-per-warp projection takes the wide walk.  Where it does not
 // fill its 64 lanes the narrow one is faster (100k queries on 100k points, 3
-// iterations but where said, narrow / wide, ms):
+// iterations but where said, narrow / wide, ms), but for calls that it holds in
+// flight at once (2,368 queries) later than for others:
 //  - its stack holds fewer ranges than the narrow walk's for twice the nodes, and
 //    near its end it pops one range a round: cutoff 6 10.3 / 9.7 and 6.6 / 6.1,
-//    9 19.3 / 23.9, 14 39 / 68; min_depth 4 9.6 / 8.3, 5 30.7 / 31.6, 6 110 / 230;
+//    9 19.3 / 23.9, 14 39 / 68; min_depth 4 9.6 / 8.3, 5 30.7 / 31.6, 6 110 / 230; 1k
+//    queries cutoff 9 0.61 / 0.44, 14 1.06 / 1.05, min_depth 5 1.00 / 0.63, 6 2.4 / 2.6;
 //  - it takes 32 of the points of a leaf of more a round: 10.2 points a node
-//    11.3 / 10.9, 15.4 11.9 / 13.9, 25 25.0 / 30.7, 87 53 / 78 -- but for calls that it
-//    holds in flight at once (2,368 queries): 25 1k queries 1.29 / 0.79, 3k 1.50 / 1.45,
-//    4k 1.69 / 1.66, 62 1k 2.27 / 1.63, 4k 2.67 / 2.95;
+//    11.3 / 10.9, 15.4 11.9 / 13.9, 25 25.0 / 30.7, 87 53 / 78; 25 1k queries 1.29 /
+//    0.79, 3k 1.50 / 1.45, 4k 1.69 / 1.66, 62 1k 2.27 / 1.63, 4k 2.67 / 2.95;
 //  - short walks spend their time in rounds of a few nodes (10 iterations):
 //    cutoff 2.5 6.0 / 6.0 and 8.4 / 7.8, 2 4.6 / 5.0 and 6.1 / 5.9, 1 3.4 / 4.4;
 //    calls of few queries, which are bound by the number of rounds, gain all the
@@ -84,8 +85,10 @@ inline bool walks_freely(const CloudArgs& c) { return c.n_iter >= 2 && !(c.prune
 // does not depend on what it is projected with, but for the number of queries.
 inline bool walks_wide(const CloudArgs& c)
 {
-    if (!walks_freely(c) || c.cutoff > 6.f || c.min_depth > 4) return false;
-    if (c.n_pts > 10 * c.n_nodes && c.n_call > 2368) return false;
+    if (!walks_freely(c)) return false;
+    const bool few = c.n_call <= 2368;
+    if (c.cutoff > (few ? 9.f : 6.f) || c.min_depth > (few ? 5 : 4)) return false;
+    if (!few && c.n_pts > 10 * c.n_nodes) return false;
     return c.cutoff >= 2.5f || c.n_call <= (c.cutoff < 2.f ? 8192 : 16384);
 }
 

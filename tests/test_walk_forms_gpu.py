@@ -34,7 +34,8 @@ def projector(pts, nrm, depth, cutoff, min_depth=0, rule=0, kind="multi", diag=N
 @pytest.mark.parametrize("n,depth,cutoff,min_depth,wide", [
     (2000, 12, 3.0, 0, True), (2000, 12, 2.0, 4, True), (40000, 12, 2.5, 0, True), (2000, 12, 6.0, 0, True),
     (16384, 12, 2.0, 0, True), (16385, 12, 2.0, 0, False), (8192, 12, 1.5, 0, True), (8193, 12, 1.5, 0, False),
-    (2000, 12, 6.5, 0, False), (2000, 12, 3.0, 5, False), (2369, 3, 3.0, 0, False)])
+    (2369, 12, 6.5, 0, False), (2369, 12, 3.0, 5, False), (2369, 3, 3.0, 0, False), (2368, 12, 6.5, 0, True),
+    (2368, 12, 9.5, 0, False), (2368, 12, 3.0, 5, True), (2368, 12, 3.0, 6, False)])
 def test_form_and_fp64(n, depth, cutoff, min_depth, wide):
     pts, nrm = synth.torus(20000, seed=31)
     pts = synth.make_tie_free(pts)
