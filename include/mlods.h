@@ -145,7 +145,9 @@ int mlods_tree_build(const float* pts, const float* nrm, int64_t n, int32_t max_
 int mlods_tree_build_device(const float* d_pts, const float* d_nrm, int64_t n, int32_t max_depth, void* stream,
                             mlods_tree* out);
 /* Frees everything the tree holds (Fastapss::eraseFromGPU + APSS::erasePointsFromGPU,
- * Fastapss.cu:486-511, GPUUtils.cu:452-464). */
+ * Fastapss.cu:486-511, GPUUtils.cu:452-464), after everything on its device has
+ * run.  The library keeps the memory for its next objects (see
+ * mlods_release_scratch). */
 int mlods_tree_free(mlods_tree t);
 int mlods_tree_get_info(mlods_tree t, mlods_tree_info* info);
 
@@ -458,7 +460,9 @@ int mlods_project_device_noalloc(mlods_tree t, int64_t n, const float* d_q, floa
  * queries per warp a request cut into pieces, which pairs its queries within
  * each piece; with one, a request large enough for mlods_project_host to walk
  * it in packets (mlods_params) cut into pieces of less than 80,000 queries or
- * two fifths of the tree's points, which are too small for that.  The
+ * two fifths of the tree's points, which are too small for that; and requests
+ * on trees of different queries_per_warp that share a batch, which runs with
+ * the larger (but for requests in packets).  The
  * query and output arrays must stay valid until the ticket is waited for.
  * Memory admission, by device footprint: a batch in flight holds, in the
  * library's stream-ordered pool, 36 bytes of query / result buffers and

@@ -5,6 +5,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <list>
+#include <map>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -145,12 +147,28 @@ struct DurableBlock {
     int device;
     unsigned long long ctx;  // a block ends with its context
 };
+// What is kept of one device's context.
+struct KeptBlocks {
+    int device;
+    unsigned long long ctx;
+    void* anchor;                  // a small block that keeps the driver's chunk for such blocks mapped
+    size_t bytes;                  // of the idle blocks
+    std::list<DurableBlock> idle;  // every use has ended; oldest first
+    std::multimap<size_t, std::list<DurableBlock>::iterator> by_size;
+};
 struct DurableState {
     std::mutex mu;
     std::unordered_map<void*, DurableBlock> live;
-    std::vector<DurableBlock> idle;   // every use has ended; oldest first
+    std::list<KeptBlocks> kept;
     std::vector<DurableBlock> stuck;  // freed, but the wait was refused
-    std::vector<DurableBlock> anchor;  // keeps the driver's chunk for small blocks mapped
+
+    KeptBlocks& of(int device, unsigned long long ctx)
+    {
+        for (KeptBlocks& k : kept)
+            if (k.device == device && k.ctx == ctx) return k;
+        kept.push_back(KeptBlocks{device, ctx, nullptr, 0, {}, {}});
+        return kept.back();
+    }
 };
 // (never destroyed: objects may be freed while the process exits)
 DurableState& durable_state()
@@ -168,21 +186,30 @@ size_t durable_size(size_t bytes)
     return (bytes + step - 1) / step * step;
 }
 
-// Takes the idle blocks of `dev` beyond `keep` bytes (the oldest) out of the list.
-std::vector<void*> take_idle(DurableState& st, int dev, unsigned long long ctx, size_t keep)
+void keep_block(KeptBlocks& k, const DurableBlock& b)
 {
-    size_t total = 0;
-    for (const DurableBlock& b : st.idle)
-        if (b.device == dev && b.ctx == ctx) total += b.size;
+    k.by_size.emplace(b.size, k.idle.insert(k.idle.end(), b));
+    k.bytes += b.size;
+}
+
+DurableBlock take_block(KeptBlocks& k, std::multimap<size_t, std::list<DurableBlock>::iterator>::iterator at)
+{
+    const DurableBlock b = *at->second;
+    k.bytes -= b.size;
+    k.idle.erase(at->second);
+    k.by_size.erase(at);
+    return b;
+}
+
+// Takes the oldest idle blocks beyond `keep` bytes.
+std::vector<void*> take_oldest(KeptBlocks& k, size_t keep)
+{
     std::vector<void*> out;
-    for (auto it = st.idle.begin(); it != st.idle.end() && total > keep;) {
-        if (it->device != dev || it->ctx != ctx) {
-            ++it;
-            continue;
-        }
-        total -= it->size;
-        out.push_back(it->p);
-        it = st.idle.erase(it);
+    while (k.bytes > keep) {
+        const auto oldest = k.idle.begin();
+        auto at = k.by_size.lower_bound(oldest->size);
+        while (at->second != oldest) ++at;
+        out.push_back(take_block(k, at).p);
     }
     return out;
 }
@@ -203,8 +230,9 @@ cudaError_t settle(DurableBlock b)
             return e;
         }
         b.fence = nullptr;
-        st.idle.push_back(b);
-        out = take_idle(st, b.device, b.ctx, kDurableKeepBytes);
+        KeptBlocks& k = st.of(b.device, b.ctx);
+        keep_block(k, b);
+        out = take_oldest(k, kDurableKeepBytes);
     }
     for (void* p : out) {
         const cudaError_t ef = cudaFree(p);
@@ -238,7 +266,7 @@ cudaError_t give_back(int dev, unsigned long long ctx)
     {
         DurableState& st = durable_state();
         std::lock_guard<std::mutex> lock(st.mu);
-        out = take_idle(st, dev, ctx, 0);
+        out = take_oldest(st.of(dev, ctx), 0);
     }
     cudaError_t e = cudaSuccess;
     for (void* p : out) {
@@ -276,13 +304,13 @@ cudaError_t durable_alloc(void** p, size_t bytes)
     cudaError_t e = cudaGetDevice(&b.device);
     if (e != cudaSuccess) return e;
     b.ctx = context_id(b.device);
-    const auto of_context = [&](const DurableBlock& o) { return o.device == b.device && o.ctx == b.ctx; };
     {
         std::lock_guard<std::mutex> lock(st.mu);
-        if (std::none_of(st.anchor.begin(), st.anchor.end(), of_context)) {
-            DurableBlock a = {nullptr, 256, nullptr, b.device, b.ctx};
-            e = cudaMalloc(&a.p, a.size);
-            if (e == cudaSuccess) st.anchor.push_back(a);
+        KeptBlocks& k = st.of(b.device, b.ctx);
+        if (!k.anchor) {
+            void* small = nullptr;
+            e = cudaMalloc(&small, 256);
+            if (e == cudaSuccess) k.anchor = small;
         }
     }
     if (e == cudaSuccess) e = cudaMalloc(&b.fence, 256);
@@ -295,15 +323,12 @@ cudaError_t durable_alloc(void** p, size_t bytes)
     settle_stuck(b.device, b.ctx);
     {
         std::lock_guard<std::mutex> lock(st.mu);
-        auto best = st.idle.end();
-        for (auto it = st.idle.begin(); it != st.idle.end(); ++it)
-            if (of_context(*it) && it->size >= bytes && it->size <= b.size + b.size / 4 &&
-                (best == st.idle.end() || it->size < best->size))
-                best = it;
-        if (best != st.idle.end()) {
-            b.p = best->p;
-            b.size = best->size;
-            st.idle.erase(best);
+        KeptBlocks& k = st.of(b.device, b.ctx);
+        const auto at = k.by_size.lower_bound(bytes);
+        if (at != k.by_size.end() && at->first <= b.size + b.size / 4) {
+            const DurableBlock kept = take_block(k, at);
+            b.p = kept.p;
+            b.size = kept.size;
         }
     }
     if (!b.p) {
@@ -365,7 +390,7 @@ cudaError_t scratch_release()
     {
         DurableState& st = durable_state();
         std::lock_guard<std::mutex> lock(st.mu);
-        held = held || !st.idle.empty() || !st.stuck.empty();
+        held = held || !st.kept.empty() || !st.stuck.empty();
     }
     if (!held) return cudaSuccess;
     e = cudaDeviceSynchronize();

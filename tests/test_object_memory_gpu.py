@@ -151,3 +151,20 @@ def test_works_on_after_a_device_reset():
     """Kept blocks and the scratch pool end with their context."""
     res = subprocess.run([sys.executable, "-c", RESET], cwd=ROOT, capture_output=True, text=True, timeout=240)
     assert res.returncode == 0, res.stderr
+
+
+def test_many_small_objects():
+    """Kept blocks are found and given up by size and age, not by a walk of all."""
+    pts, nrm = synth.torus(64, seed=11)
+    pts = synth.make_tie_free(pts)
+    torch.cuda.synchronize()
+    for _ in range(2):
+        trees = []
+        for _ in range(300):
+            t = APSSOctree()
+            t.build(pts, nrm)
+            trees.append(t)
+        assert len({t.nbOfNodes() for t in trees}) == 1
+        for t in trees:
+            t.free()
+    capi.check(capi.load().mlods_release_scratch())
