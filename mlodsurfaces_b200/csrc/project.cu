@@ -957,7 +957,7 @@ struct WarpTotals {
     }
     __device__ void flush(int64_t* stats)
     {
-        if ((threadIdx.x & 31) != 0 || !stats) return;
+        if ((threadIdx.x & 31) != 0 || !stats || iterations == 0) return;
         atomicAdd(reinterpret_cast<unsigned long long*>(&stats[0]), (unsigned long long)visits);
         atomicAdd(reinterpret_cast<unsigned long long*>(&stats[4]), (unsigned long long)rounds);
         atomicAdd(reinterpret_cast<unsigned long long*>(&stats[5]), (unsigned long long)iterations);
